@@ -23,6 +23,7 @@
 
 #include "../../include/granb200.h"
 #include "gb2_mlp.cuh"
+#include "gb2_sq_solve.cuh"
 
 using namespace gb2;
 using namespace gb2::sq;
@@ -247,6 +248,7 @@ struct gb2_sq_ctx {
     // counts and the taken counter
     Buf<int> work;
     Buf<signed char> kind;   // per slot: the work list the screen puts it on
+    Buf<float4> guess;       // learned guesses of the first contacts, by list position
     int nsm = 148;
 };
 
@@ -468,10 +470,17 @@ int sq_force(gb2_sq_ctx *c, int shearupdate)
             SQCK(cub::DeviceSelect::If(c->tmp.p, bytes, slots, W.list[l], W.n + l, (int)ns,
                                        SlotKindIs{c->kind.p, (signed char)l}, c->st));
         }
-        // the solves: enough resident warps to fill the GPU; each warp takes
-        // the next 32 items (first contacts, then warm starts) until none
+        const float4 *guess = nullptr;
+        if (D.mlp) {   // the learned guesses of the first contacts, one block per SM at most
+            SQCK(c->guess.alloc(ns));
+            k_sq_guess<<<std::min(c->nsm, nb((long)ns)), kB, 0, c->st>>>(D, W, c->own.p, c->guess.p);
+            SQCKL();
+            guess = c->guess.p;
+        }
+        // the solves, eight lanes each: as many groups as stay resident, each
+        // taking the next item (first contacts, then warm starts) until none
         // are left
-        k_sq_solve<<<2 * c->nsm, kB, 0, c->st>>>(D, W, c->own.p, shearupdate);
+        k_sq_solve<<<3 * c->nsm, kB, 0, c->st>>>(D, W, c->own.p, shearupdate, guess);
         SQCKL();
     }
     k_sq_sum<<<nb(c->n), kB, 0, c->st>>>(D);

@@ -5,9 +5,7 @@
 // (src/superquadric.cpp:111-330), the 4-unknown Newton solve for the contact
 // point with golden-section fallback (src/math_extra_liggghts_superquadric.cpp:778-1020),
 // the sphere-to-shape homotopy for pairs without a previous point (:1391),
-// the oriented-box pre-test (:166), the line-surface intersection that
-// measures the overlap (src/superquadric.cpp:712-818, extended overlap :1489)
-// and the asphere integrator (src/fix_nve_asphere_base.cpp:319-620,
+// the oriented-box pre-test (:166) and the asphere integrator (src/fix_nve_asphere_base.cpp:319-620,
 // integration_scheme 1).  The arithmetic is FP64 throughout; pow() with a
 // non-integer exponent comes from CUDA's math library, so results agree
 // with the CPU restatement to the solver tolerance, not bit for bit.
@@ -131,41 +129,6 @@ __device__ __forceinline__ void to_local(const Body &b, const double *x, double 
 {
     const double t[3] = {x[0] - b.c[0], x[1] - b.c[1], x[2] - b.c[2]};
     tmatvec(b.rot, t, xl);
-}
-
-// shape function value in the body frame (Superquadric::shape_function_local)
-__device__ __forceinline__ double f_local(const Body &b, const double *xl)
-{
-    double f;
-    if (b.use_int) {
-        const int ni = (int)floor(b.n + 1e-2);
-        f = pow_abs_int(xl[0] * b.inv[0], ni) + pow_abs_int(xl[1] * b.inv[1], ni) + pow_abs_int(xl[2] * b.inv[2], ni) -
-            1.0;
-    } else {
-        f = (pow_abs(pow_abs(xl[0] * b.inv[0], b.n) + pow_abs(xl[1] * b.inv[1], b.n), 1.0) +
-             pow_abs(xl[2] * b.inv[2], b.n) - 1.0);
-    }
-    return b.koef * f;
-}
-
-__device__ __forceinline__ void grad_local(const Body &b, const double *xl, double *g)
-{
-    const double a = b.inv[0], bb = b.inv[1], c = b.inv[2], n = b.n;
-    const double xa = xl[0] * a, yb = xl[1] * bb, zc = xl[2] * c;
-    double xan21, ybn21, zcn11;
-    if (b.use_int) {
-        const int ni = (int)floor(n + 1e-2);
-        xan21 = pow_abs_int(xa, ni - 1);
-        ybn21 = pow_abs_int(yb, ni - 1);
-        zcn11 = pow_abs_int(zc, ni - 1);
-    } else {
-        xan21 = pow_abs(xa, n - 1.0);
-        ybn21 = pow_abs(yb, n - 1.0);
-        zcn11 = pow_abs(zc, n - 1.0);
-    }
-    g[0] = n * (b.koef * a) * sgn(xa) * xan21;
-    g[1] = n * (b.koef * bb) * sgn(yb) * ybn21;
-    g[2] = n * (b.koef * c) * sgn(zc) * zcn11;
 }
 
 // value, gradient and (optionally) Hessian in the global frame
@@ -508,84 +471,6 @@ __device__ __forceinline__ bool obb_intersect(const double *ca, const double *Ra
             if (fabs(TA[i2] * C[3 * i1 + j] - TA[i1] * C[3 * i2 + j]) > ra + rb) return false;
         }
     return true;
-}
-
-// Superquadric::surface_line_intersection with 20 iterations: the parameter
-// alpha where start + alpha * dir meets the surface (Newton with halving)
-__device__ __forceinline__ double line_intersection(const Body &b, const double *start, const double *dir,
-                                                    double alpha_prev, double *result)
-{
-    double sl[3], dl[3], point[3], gl[3];
-    to_local(b, start, sl);
-    tmatvec(b.rot, dir, dl);
-    double alpha = alpha_prev;
-    const double eps0 = 1e-14;
-    if (comp_double(b.n, 2.0, 1e-2)) {
-        const double x0 = sl[0] * b.inv[0], nx = dl[0] * b.inv[0];
-        const double y0 = sl[1] * b.inv[1], ny = dl[1] * b.inv[1];
-        const double z0 = sl[2] * b.inv[2], nz = dl[2] * b.inv[2];
-        const double qa = nx * nx + ny * ny + nz * nz, qb = 2.0 * (x0 * nx + y0 * ny + z0 * nz);
-        const double qc = x0 * x0 + y0 * y0 + z0 * z0 - 1.0;
-        const double D = qb * qb - 4.0 * qa * qc, tai = 0.5 / qa;
-        double a1, a2;
-        if (D < 0) {
-            a1 = -qb * tai;
-            a2 = a1;
-        } else {
-            const double sD = sqrt(D);
-            a1 = (-qb + sD) * tai;
-            a2 = (-qb - sD) * tai;
-        }
-        if (a1 > -eps0 && a2 < -eps0) alpha = a1;
-        else if (a1 < -eps0 && a2 > -eps0) alpha = a2;
-        else if (a1 < -eps0 && a2 < -eps0) alpha = fmax(a1, a2);
-        else alpha = fmin(a1, a2);
-    } else {
-        const double a = 0.5 * fmin(fmin(b.shape[0], b.shape[1]), b.shape[2]) / sqrt(dot3(dir, dir));
-        const double eps = 1e-16;
-        alpha = alpha < -a ? -a : (alpha > a ? a : alpha);
-        for (int k = 0; k < 3; k++) point[k] = sl[k] + alpha * dl[k];
-        double f0 = f_local(b, point);
-        if (!(fabs(f0) < eps)) {
-            for (int it = 0; it < 20; it++) {
-                if (fabs(f0) < eps * b.koef) break;
-                grad_local(b, point, gl);
-                const double f_der = dot3(gl, dl);
-                double delta;
-                if (fabs(f_der) < 1e-10) {
-                    delta = 1e-10;
-                    double p_[3], g_[3];
-                    for (int k = 0; k < 3; k++) p_[k] = point[k] + delta * dl[k];
-                    grad_local(b, p_, g_);
-                    if (dot3(g_, dl) < 0.0) delta = -delta;
-                } else {
-                    delta = -f0 / f_der;
-                    delta = delta < -a ? -a : (delta > a ? a : delta);
-                }
-                if (fabs(delta) <= eps) {
-                    alpha += delta;
-                    for (int k = 0; k < 3; k++) point[k] = point[k] + delta * dl[k];
-                    break;
-                }
-                int halvings = 0;
-                while (fabs(delta) > eps && halvings < 80) {
-                    double p_[3];
-                    for (int k = 0; k < 3; k++) p_[k] = point[k] + delta * dl[k];
-                    const double f_ = f_local(b, p_);
-                    if (fabs(f_) < fabs(f0) || fabs(f_) < eps * b.koef) {
-                        f0 = f_;
-                        alpha += delta;
-                        for (int k = 0; k < 3; k++) point[k] = p_[k];
-                        break;
-                    }
-                    delta *= 0.5;
-                    halvings++;
-                }
-            }
-        }
-    }
-    for (int k = 0; k < 3; k++) result[k] = start[k] + alpha * dir[k];
-    return alpha;
 }
 
 // FixNVEAsphereBase, integration_scheme 1 helpers (src/math_extra.h, src/math_extra_liggghts_nonspherical.cpp:175)
