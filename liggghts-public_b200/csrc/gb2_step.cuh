@@ -95,10 +95,6 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
     const int tkk = D.type[kk], to = D.type[other];
     // material lookup in the reference's (owner, neighbour) order
     const MatPair &M = own ? mat(D, tkk, to) : mat(D, to, tkk);
-    if (own) {
-        const int fl = D.flag[e];
-        if ((fl | 5) != fl) D.flag[e] = fl | 5;   // CONTACT_NORMAL_MODEL | CONTACT_TANGENTIAL_MODEL
-    }
     if constexpr (SPLIT) {
         const flt8 a = ldg8f(&D.kin[kk]), b = ldg8f(&D.kin[other]);
         const double r = sqrt(rsq);
@@ -287,13 +283,17 @@ static __global__ void k_stream_positions(Dev D)
     if (stream_hold(D, i, x, v, w)) D.pos[i] = x;
 }
 
-// Shear of own slots that stopped touching this step is carried into the
-// write buffer, and the touching mask is kept for the next step.
+// Own slots that touch and did not in the previous step (prevm; empty after
+// a build and in setup) get their contact flag; shear of own slots that
+// stopped touching is carried into the write buffer, and the touching mask is
+// kept for the next step.
 __device__ __forceinline__ void atom_hist_tail(const Dev &D, int k, unsigned long long prevm,
                                                unsigned long long mown, bool upd)
 {
-    if (!upd) return;
     const int cap = D.cap;
+    for (unsigned long long fresh = mown & ~prevm; fresh; fresh &= fresh - 1ull)
+        D.flag[(__ffsll((long long)fresh) - 1) * cap + k] |= 5;   // CONTACT_NORMAL_MODEL | CONTACT_TANGENTIAL_MODEL
+    if (!upd) return;
     unsigned long long stopped = prevm & ~mown;
     while (stopped) {
         const int s = __ffsll((long long)stopped) - 1;
