@@ -181,7 +181,8 @@ struct gb2_ctx {
     DBuf<int> nnum, nbr, flag, rnum, rev, pnum, ptag, tail;
     DBuf<int> type_s, tag_s, pnum_s, ptag_s;   // atom-sort shadows
     DBuf<double> phist_s;
-    DBuf<double> hist, hist2, phist;
+    DBuf<dbl4> hist, hist2;
+    DBuf<double> phist;
     DBuf<unsigned long long> prevmask;
     DBuf<int> gsrc;
     DBuf<dbl4> gshift;
@@ -1042,8 +1043,8 @@ int do_build(gb2_ctx *c)
         c->maxn = grown_capacity(c, 0, c->maxn, 256);
         CK(c->nbr.alloc((size_t)c->maxn * c->cap));
         CK(c->flag.alloc((size_t)c->maxn * c->cap));
-        CK(c->hist.alloc((size_t)3 * c->maxn * c->cap));
-        CK(c->hist2.alloc((size_t)3 * c->maxn * c->cap));
+        CK(c->hist.alloc((size_t)c->maxn * c->cap));
+        CK(c->hist2.alloc((size_t)c->maxn * c->cap));
         if (attempt == 7) return set_err(c, GB2_ERR_CAPACITY, "neighbor list capacity could not be grown");
     }
     for (int attempt = 0; attempt < 8; attempt++) {
@@ -1524,8 +1525,8 @@ int gb2_upload_atoms(gb2_ctx *c, int n, const double *x, const double *v, const 
     CK(c->pnum.alloc(cap));
     CK(c->nbr.alloc((size_t)c->maxn * cap));
     CK(c->flag.alloc((size_t)c->maxn * cap));
-    CK(c->hist.alloc((size_t)3 * c->maxn * cap));
-    CK(c->hist2.alloc((size_t)3 * c->maxn * cap));
+    CK(c->hist.alloc((size_t)c->maxn * cap));
+    CK(c->hist2.alloc((size_t)c->maxn * cap));
     CK(c->prevmask.alloc(cap));
     CK(c->rev.alloc((size_t)c->maxr * cap));
     CK(c->revs.alloc((size_t)c->maxr * cap));
@@ -1742,8 +1743,8 @@ static int reserve_cap(gb2_ctx *c, int want)
     CK(c->pnum.alloc(cap));
     CK(c->nbr.alloc((size_t)c->maxn * cap));
     CK(c->flag.alloc((size_t)c->maxn * cap));
-    CK(c->hist.alloc((size_t)3 * c->maxn * cap));
-    CK(c->hist2.alloc((size_t)3 * c->maxn * cap));
+    CK(c->hist.alloc((size_t)c->maxn * cap));
+    CK(c->hist2.alloc((size_t)c->maxn * cap));
     CK(c->prevmask.alloc(cap));
     CK(c->rev.alloc((size_t)c->maxr * cap));
     CK(c->revs.alloc((size_t)c->maxr * cap));
@@ -2473,11 +2474,11 @@ int gb2_download_pairs(gb2_ctx *c, int cap, int *n, int *tag_i, int *tag_j, int 
     const size_t cp = c->cap;
     const int nl = c->nlocal;
     std::vector<int> nnum(nl), nbr((size_t)c->maxn * cp), fl((size_t)c->maxn * cp), tg(c->nlocal + c->nghost);
-    std::vector<double> h((size_t)3 * c->maxn * cp);
+    std::vector<dbl4> h((size_t)c->maxn * cp);
     CK(cudaMemcpyAsync(nnum.data(), c->nnum.p, sizeof(int) * nl, cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(nbr.data(), c->nbr.p, sizeof(int) * nbr.size(), cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(fl.data(), c->flag.p, sizeof(int) * fl.size(), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(h.data(), c->hist.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(h.data(), c->hist.p, sizeof(dbl4) * h.size(), cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(tg.data(), c->tag.p, sizeof(int) * tg.size(), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     int k = 0;
@@ -2488,8 +2489,11 @@ int gb2_download_pairs(gb2_ctx *c, int cap, int *n, int *tag_i, int *tag_j, int 
                 if (tag_i) tag_i[k] = tg[i];
                 if (tag_j) tag_j[k] = tg[nbr[e]];
                 if (flag) flag[k] = fl[e];
-                if (hist)
-                    for (int q = 0; q < 3; q++) hist[3 * k + q] = h[(size_t)(3 * s + q) * cp + i];
+                if (hist) {
+                    hist[3 * k] = h[e].x;
+                    hist[3 * k + 1] = h[e].y;
+                    hist[3 * k + 2] = h[e].z;
+                }
             }
             k++;
         }

@@ -14,7 +14,8 @@
 //   half neighbour list, slot-major so a warp reads consecutive atoms
 //   (capacity maxn slots per owned atom, stride `cap`):
 //     nnum[i], nbr[s*cap+i] (j index), flag[s*cap+i] (contact flag bits),
-//     hist[(3s+c)*cap+i] (shear history, FP64)
+//     hist[s*cap+i] {s0, s1, s2, -} (shear history, FP64: one 32-byte
+//     sector, so the j side's scattered read of a slot is one sector, not three)
 //   reverse list (entries where the atom is the j side, ascending owner):
 //     rnum[k], rev[r*cap+k] = owner i', revs[r*cap+k] = its slot s'
 //   contact-history partners (FixContactHistory::partner_, keyed by tag):
@@ -131,8 +132,8 @@ struct Dev {
     int maxn;
     int item_cap;          // per-warp list capacity of the pair step's listed rounds (<= kItemCap)
     int *nnum, *nbr, *flag;
-    double *hist;          // shear read buffer (current values)
-    double *hist_out;      // shear write buffer of the pair step
+    dbl4 *hist;            // shear read buffer (current values)
+    dbl4 *hist_out;        // shear write buffer of the pair step
     unsigned long long *prevmask;   // own slots touching in the previous step
     // reverse list
     int maxr;

@@ -152,7 +152,10 @@ __global__ void k_partners(Dev D)
         if (!D.flag[s * cap + i]) continue;
         if (np < D.maxp) {
             D.ptag[np * cap + k] = D.tag[i];
-            for (int c = 0; c < 3; c++) D.phist[(3 * np + c) * cap + k] = -D.hist[(3 * s + c) * cap + i];
+            const dbl4 h = D.hist[s * cap + i];
+            D.phist[(3 * np + 0) * cap + k] = -h.x;
+            D.phist[(3 * np + 1) * cap + k] = -h.y;
+            D.phist[(3 * np + 2) * cap + k] = -h.z;
         }
         np++;
     }
@@ -162,7 +165,10 @@ __global__ void k_partners(Dev D)
         if (!D.flag[e]) continue;
         if (np < D.maxp) {
             D.ptag[np * cap + k] = D.tag[D.nbr[e]];
-            for (int c = 0; c < 3; c++) D.phist[(3 * np + c) * cap + k] = D.hist[(3 * s + c) * cap + k];
+            const dbl4 h = D.hist[e];
+            D.phist[(3 * np + 0) * cap + k] = h.x;
+            D.phist[(3 * np + 1) * cap + k] = h.y;
+            D.phist[(3 * np + 2) * cap + k] = h.z;
         }
         np++;
     }
@@ -361,12 +367,7 @@ __global__ void k_build_list(Dev D)
                     }
                     D.flag[e] = fl;
                     // both history buffers, so either can serve as the next read buffer
-                    D.hist[(3 * n + 0) * cap + i] = h0;
-                    D.hist[(3 * n + 1) * cap + i] = h1;
-                    D.hist[(3 * n + 2) * cap + i] = h2;
-                    D.hist_out[(3 * n + 0) * cap + i] = h0;
-                    D.hist_out[(3 * n + 1) * cap + i] = h1;
-                    D.hist_out[(3 * n + 2) * cap + i] = h2;
+                    D.hist[e] = D.hist_out[e] = dbl4{h0, h1, h2, 0.0};
                 }
                 n++;
             }
@@ -1070,7 +1071,8 @@ __global__ void k_pgl_rows(Dev D, const int *off, double *rows, PglBox B, unsign
         if (!pgl_pair(D, i, s, pi, j, delx, dely, delz, rsq)) continue;
         const dbl4 pj = D.pos[j], vj4 = D.vel[j], wj4 = D.omg[j];
         const double vj[3] = {vj4.x, vj4.y, vj4.z}, wj[3] = {wj4.x, wj4.y, wj4.z};
-        double sh[3] = {D.hist[(3 * s + 0) * cap + i], D.hist[(3 * s + 1) * cap + i], D.hist[(3 * s + 2) * cap + i]};
+        const dbl4 h4 = D.hist[s * cap + i];
+        double sh[3] = {h4.x, h4.y, h4.z};
         const double h0[3] = {sh[0], sh[1], sh[2]};
         ContactOut o;
         pair_contact<false>(mat(D, ti, D.type[j]), delx, dely, delz, rsq, pi.w, pj.w, vi, vj, wi, wj, vi4.w, vj4.w,

@@ -29,10 +29,8 @@ __device__ __forceinline__ void serial_atom(const Dev &D, int k, const dbl4 &pk,
         const int s = D.revs[r * cap + k];
         const dbl4 v4 = ldg4(&D.vel[i]), w4 = ldg4(&D.omg[i]);
         const double vi[3] = {v4.x, v4.y, v4.z}, wi[3] = {w4.x, w4.y, w4.z};
-        double sh[3];
-        sh[0] = -D.hist[(3 * s + 0) * cap + i];
-        sh[1] = -D.hist[(3 * s + 1) * cap + i];
-        sh[2] = -D.hist[(3 * s + 2) * cap + i];
+        const dbl4 h = ldg4(&D.hist[s * cap + i]);
+        double sh[3] = {-h.x, -h.y, -h.z};
         pair_contact(mat(D, D.type[i], tk), delx, dely, delz, rsq, pk.w, pi.w, vk, vi, wk, wi, vi4.w, v4.w, sh,
                      upd, D.dt, ROLLING, D.tdamp != 0, acc);
     }
@@ -45,8 +43,8 @@ __device__ __forceinline__ void serial_atom(const Dev &D, int k, const dbl4 &pk,
         const double delz = pk.z - pj.z;
         const double rsq = delx * delx + dely * dely + delz * delz;
         const double radsum = pk.w + pj.w;
-        double sh[3] = {D.hist[(3 * s + 0) * cap + k], D.hist[(3 * s + 1) * cap + k],
-                        D.hist[(3 * s + 2) * cap + k]};
+        const dbl4 h = ldg4(&D.hist[e]);
+        double sh[3] = {h.x, h.y, h.z};
         if (rsq < radsum * radsum) {
             const dbl4 v4 = ldg4(&D.vel[j]), w4 = ldg4(&D.omg[j]);
             const double vj[3] = {v4.x, v4.y, v4.z}, wj[3] = {w4.x, w4.y, w4.z};
@@ -55,11 +53,7 @@ __device__ __forceinline__ void serial_atom(const Dev &D, int k, const dbl4 &pk,
             pair_contact(mat(D, tk, D.type[j]), delx, dely, delz, rsq, pk.w, pj.w, vk, vj, wk, wj, vi4.w, v4.w,
                          sh, upd, D.dt, ROLLING, D.tdamp != 0, acc);
         }
-        if (upd) {   // serial atoms write every slot
-            D.hist_out[(3 * s + 0) * cap + k] = sh[0];
-            D.hist_out[(3 * s + 1) * cap + k] = sh[1];
-            D.hist_out[(3 * s + 2) * cap + k] = sh[2];
-        }
+        if (upd) D.hist_out[e] = dbl4{sh[0], sh[1], sh[2], 0.0};   // serial atoms write every slot
     }
 }
 
@@ -102,18 +96,12 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
         const float va[3] = {a.vx, a.vy, a.vz}, wa[3] = {a.wx, a.wy, a.wz};
         const float vb[3] = {b.vx, b.vy, b.vz}, wb[3] = {b.wx, b.wy, b.wz};
         const float fs = (float)sgn;
-        float sh[3];
-        sh[0] = fs * (float)D.hist[(3 * s + 0) * cap + hrow];
-        sh[1] = fs * (float)D.hist[(3 * s + 1) * cap + hrow];
-        sh[2] = fs * (float)D.hist[(3 * s + 2) * cap + hrow];
+        const dbl4 h = ldg4(&D.hist[s * cap + hrow]);
+        float sh[3] = {fs * (float)h.x, fs * (float)h.y, fs * (float)h.z};
         ContactOutF o;
         pair_contact_f32(M, (float)delx, (float)dely, (float)delz, (float)r, (float)deltan, (float)pkk.w,
                          (float)po.w, va, vb, wa, wb, a.m, b.m, sh, upd, (float)D.dt, ROLLING, D.tdamp != 0, o);
-        if (own && upd) {
-            D.hist_out[(3 * s + 0) * cap + kk] = sh[0];
-            D.hist_out[(3 * s + 1) * cap + kk] = sh[1];
-            D.hist_out[(3 * s + 2) * cap + kk] = sh[2];
-        }
+        if (own && upd) D.hist_out[e] = dbl4{(double)sh[0], (double)sh[1], (double)sh[2], 0.0};
         for (int c = 0; c < 3; c++) {
             res[c] = o.F[c];
             res[3 + c] = o.T[c];
@@ -123,18 +111,12 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
         const dbl4 vo4 = ldg4(&D.vel[other]), wo4 = ldg4(&D.omg[other]);
         const double vk[3] = {vk4.x, vk4.y, vk4.z}, wk[3] = {wk4.x, wk4.y, wk4.z};
         const double vo[3] = {vo4.x, vo4.y, vo4.z}, wo[3] = {wo4.x, wo4.y, wo4.z};
-        double sh[3];
-        sh[0] = sgn * D.hist[(3 * s + 0) * cap + hrow];   // exact: multiplying by +-1 only flips the sign
-        sh[1] = sgn * D.hist[(3 * s + 1) * cap + hrow];
-        sh[2] = sgn * D.hist[(3 * s + 2) * cap + hrow];
+        const dbl4 h = ldg4(&D.hist[s * cap + hrow]);
+        double sh[3] = {sgn * h.x, sgn * h.y, sgn * h.z};   // exact: multiplying by +-1 only flips the sign
         ContactOut o;
         pair_contact<false>(M, delx, dely, delz, rsq, pkk.w, po.w, vk, vo, wk, wo, vk4.w, vo4.w, sh, upd, D.dt,
                             ROLLING, D.tdamp != 0, o);
-        if (own && upd) {
-            D.hist_out[(3 * s + 0) * cap + kk] = sh[0];
-            D.hist_out[(3 * s + 1) * cap + kk] = sh[1];
-            D.hist_out[(3 * s + 2) * cap + kk] = sh[2];
-        }
+        if (own && upd) D.hist_out[e] = dbl4{(double)sh[0], (double)sh[1], (double)sh[2], 0.0};
         for (int c = 0; c < 3; c++) {
             res[c] = o.F[c];
             res[3 + c] = o.T[c];
@@ -298,9 +280,7 @@ __device__ __forceinline__ void atom_hist_tail(const Dev &D, int k, unsigned lon
     while (stopped) {
         const int s = __ffsll((long long)stopped) - 1;
         stopped &= stopped - 1ull;
-        D.hist_out[(3 * s + 0) * cap + k] = D.hist[(3 * s + 0) * cap + k];
-        D.hist_out[(3 * s + 1) * cap + k] = D.hist[(3 * s + 1) * cap + k];
-        D.hist_out[(3 * s + 2) * cap + k] = D.hist[(3 * s + 2) * cap + k];
+        D.hist_out[s * cap + k] = ldg4(&D.hist[s * cap + k]);
     }
     D.prevmask[k] = mown;
 }
