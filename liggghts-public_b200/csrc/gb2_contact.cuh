@@ -21,6 +21,9 @@ namespace gb2 {
 // MODEL_PARAMS::createYeff/createGeff/createBetaEff do
 struct MatPair {
     double Yeff, Geff, betaeff, mu, mur;
+    // the products that open the model's expressions, rounded as it rounds them:
+    // 2 Yeff, 8 Geff, 4/3 Yeff, -2 sqrt(5/6) betaeff
+    double Y2, G8, Y43, b56;
 };
 
 struct ContactOut {
@@ -28,10 +31,10 @@ struct ContactOut {
     double T[3];
 };
 
-#ifdef __CUDACC__   // device code; host-only units see the structs
-
 // sqrt(5/6) as written in src/normal_model_hertz.h:235
 #define GB2_SQRT_FIVE_OVER_SIX 0.91287092917527685576161630466800355658790782499663875
+
+#ifdef __CUDACC__   // device code; host-only units see the structs
 
 // One sphere-sphere contact seen from particle "i" (the half-list owner in
 // the reference, or the j-particle when a reverse entry is evaluated from
@@ -79,12 +82,12 @@ __device__ __forceinline__ void pair_contact(const MatPair &M, double delx, doub
     // ---- normal model (Hertz)
     const double reff = radi * radj / (radi + radj);
     const double sqrtval = sqrt(reff * deltan);
-    const double Sn = 2. * M.Yeff * sqrtval;
-    const double St = 8. * M.Geff * sqrtval;
-    double kn = 4. / 3. * M.Yeff * sqrtval;
+    const double Sn = M.Y2 * sqrtval;
+    const double St = M.G8 * sqrtval;
+    double kn = M.Y43 * sqrtval;
     double kt = St;
-    const double gamman = -2. * GB2_SQRT_FIVE_OVER_SIX * M.betaeff * sqrt(Sn * meff);
-    const double gammat = tdamp ? -2. * GB2_SQRT_FIVE_OVER_SIX * M.betaeff * sqrt(St * meff) : 0.0;
+    const double gamman = M.b56 * sqrt(Sn * meff);
+    const double gammat = tdamp ? M.b56 * sqrt(St * meff) : 0.0;
     kn /= 1.0;   // force->nktv2p = 1 (si)
     kt /= 1.0;
     const double Fn_damping = -gamman * vn;
@@ -346,12 +349,12 @@ __device__ __forceinline__ void wall_contact(const MatPair &M, const double d[3]
     // ---- normal model, wall branch (reff = radi, meff = particle mass)
     const double reff = radi;
     const double sqrtval = sqrt(reff * deltan);
-    const double Sn = 2. * M.Yeff * sqrtval;
-    const double St = 8. * M.Geff * sqrtval;
-    double kn = 4. / 3. * M.Yeff * sqrtval;
+    const double Sn = M.Y2 * sqrtval;
+    const double St = M.G8 * sqrtval;
+    double kn = M.Y43 * sqrtval;
     double kt = St;
-    const double gamman = -2. * GB2_SQRT_FIVE_OVER_SIX * M.betaeff * sqrt(Sn * mass);
-    const double gammat = tdamp ? -2. * GB2_SQRT_FIVE_OVER_SIX * M.betaeff * sqrt(St * mass) : 0.0;
+    const double gamman = M.b56 * sqrt(Sn * mass);
+    const double gammat = tdamp ? M.b56 * sqrt(St * mass) : 0.0;
     kn /= 1.0;
     kt /= 1.0;
     const double Fn_damping = -gamman * vn;

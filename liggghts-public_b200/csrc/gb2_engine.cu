@@ -427,6 +427,7 @@ Dev make_dev(gb2_ctx *c)
     D.bin_start = c->bin_start.p;
     D.bin_atoms = c->bin_atoms.p;
     D.mat = c->dmat.p;
+    D.mat1 = c->hmat[(kMaxTypes + 1) + 1];
     D.ntypes = c->P.ntypes;
     D.dt = c->P.dt;
     D.skin = c->P.skin;
@@ -1211,8 +1212,8 @@ int adapt_item_cap(gb2_ctx *c)
 template <bool R, int MINB>
 void launch_pair_kernel(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int fuse_next, int store_f)
 {
-    k_pair_step<R, MINB, false><<<nblk(c->nlocal), kBlock, pair_list_smem(c), c->st>>>(D, shearupdate, integrate,
-                                                                                     fuse_next, store_f);
+    const auto kernel = D.ntypes == 1 ? k_pair_step<R, MINB, false, true> : k_pair_step<R, MINB, false, false>;
+    kernel<<<nblk(c->nlocal), kBlock, pair_list_smem(c), c->st>>>(D, shearupdate, integrate, fuse_next, store_f);
 }
 
 // The pair step kernel of one time step (every atom's pair sums; the
@@ -1229,12 +1230,10 @@ void launch_pair(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int f
     // packed 1M hopper, ahead of 4 (128) and 6 (80)
     const int mb = c->minb ? c->minb : 5;
     if (c->P.rolling_cdt) {
-        if (mb == 4) launch_pair_kernel<true, 4>(c, D, shearupdate, integrate, fuse_next, store_f);
-        else if (mb == 5) launch_pair_kernel<true, 5>(c, D, shearupdate, integrate, fuse_next, store_f);
+        if (mb == 5) launch_pair_kernel<true, 5>(c, D, shearupdate, integrate, fuse_next, store_f);
         else launch_pair_kernel<true, 6>(c, D, shearupdate, integrate, fuse_next, store_f);
     } else {
-        if (mb == 4) launch_pair_kernel<false, 4>(c, D, shearupdate, integrate, fuse_next, store_f);
-        else if (mb == 5) launch_pair_kernel<false, 5>(c, D, shearupdate, integrate, fuse_next, store_f);
+        if (mb == 5) launch_pair_kernel<false, 5>(c, D, shearupdate, integrate, fuse_next, store_f);
         else launch_pair_kernel<false, 6>(c, D, shearupdate, integrate, fuse_next, store_f);
     }
 }
@@ -1464,6 +1463,10 @@ int gb2_set_materials(gb2_ctx *c, const double *youngs, const double *poisson, c
             m.betaeff = lg / std::sqrt(std::pow(lg, 2.) + std::pow(M_PI, 2.));
             m.mu = friction[(i - 1) * nt + (j - 1)];
             m.mur = rollfriction ? rollfriction[(i - 1) * nt + (j - 1)] : 0.0;
+            m.Y2 = 2. * m.Yeff;
+            m.G8 = 8. * m.Geff;
+            m.Y43 = 4. / 3. * m.Yeff;
+            m.b56 = -2. * GB2_SQRT_FIVE_OVER_SIX * m.betaeff;
         }
     if (c->dmat.alloc((kMaxTypes + 1) * (kMaxTypes + 1))) return set_err(c, GB2_ERR_CUDA, "alloc");
     CK(cudaMemcpyAsync(c->dmat.p, c->hmat, sizeof c->hmat, cudaMemcpyHostToDevice, c->st));

@@ -158,6 +158,7 @@ struct Dev {
     // materials [(kMaxTypes+1)^2]
     const MatPair *mat;
     int ntypes;
+    MatPair mat1;            // the only pair when ntypes is 1: read as launch constants
     // physics
     double dt, skin, cutneighmax, triggersq;
     int rolling, tdamp;

@@ -73,7 +73,7 @@ __device__ __forceinline__ bool step_cancelled(const Dev &D) { return D.dstop &&
 // list otherwise).  A j-side entry is evaluated from kk's side with the
 // shear negated; an own entry updates kk's shear slot in the write buffer
 // and sets the contact flag.  res receives the pair's force and torque on kk.
-template <bool ROLLING, bool SPLIT, typename Real>
+template <bool ROLLING, bool SPLIT, bool ONE, typename Real>
 __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s, bool own, bool upd, Real *res)
 {
     const int cap = D.cap;
@@ -86,9 +86,8 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
     const double dely = pkk.y - po.y;
     const double delz = pkk.z - po.z;
     const double rsq = delx * delx + dely * dely + delz * delz;
-    const int tkk = D.type[kk], to = D.type[other];
     // material lookup in the reference's (owner, neighbour) order
-    const MatPair &M = own ? mat(D, tkk, to) : mat(D, to, tkk);
+    const MatPair &M = ONE ? D.mat1 : (own ? mat(D, D.type[kk], D.type[other]) : mat(D, D.type[other], D.type[kk]));
     if constexpr (SPLIT) {
         const flt8 a = ldg8f(&D.kin[kk]), b = ldg8f(&D.kin[other]);
         const double r = sqrt(rsq);
@@ -327,7 +326,7 @@ __device__ __forceinline__ void atom_fix_tail(const Dev &D, int k, const dbl4 &p
 // shared memory, and summed by each owner lane in that order.  Atoms with
 // more than 64 reverse or own entries are evaluated serially by their owner
 // lane after the rounds, in the same order.
-template <bool ROLLING, int MINB, bool SPLIT>
+template <bool ROLLING, int MINB, bool SPLIT, bool ONE>
 __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate, int integrate, int fuse_next,
                                                          int store_f)
 {
@@ -352,7 +351,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     const bool upd = shearupdate != 0;
     dbl4 pk;
     unsigned long long prevm = 0ull;
-    int nr = 0, nn = 0, tk = 0;
+    int nr = 0, nn = 0;
     unsigned long long mrev = 0ull, mown = 0ull;
     bool serial = false, tail = false;
     if (valid) {
@@ -364,7 +363,6 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
         pk = D.pos[k];
         nr = D.rnum[k];
         nn = D.nnum[k];
-        tk = D.type[k];
         serial = nr > 64 || nn > 64;
         tail = tail_atom(D, k, nr, nn);
         if (!serial && upd) prevm = D.prevmask[k];
@@ -398,7 +396,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
                     const int2 item = (li ? lown : lrev)[w];
                     L = item.y & 31;
                     Real res[6];
-                    eval_item<ROLLING, SPLIT>(D, wbase + L, item.x, item.y >> 8, li == 1, upd, res);
+                    eval_item<ROLLING, SPLIT, ONE>(D, wbase + L, item.x, item.y >> 8, li == 1, upd, res);
 #pragma unroll
                     for (int c = 0; c < 6; c++) sres[wid][lane][c] = res[c];
                 }
@@ -442,7 +440,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
                     own = true;
                 }
                 Real res[6];
-                eval_item<ROLLING, SPLIT>(D, kk, other, s, own, upd, res);
+                eval_item<ROLLING, SPLIT, ONE>(D, kk, other, s, own, upd, res);
 #pragma unroll
                 for (int c = 0; c < 6; c++) sres[wid][lane][c] = res[c];
             }
