@@ -14,6 +14,9 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#ifdef __CUDACC__
+#include "gb2_fastmath.cuh"
+#endif
 
 namespace gb2 {
 
@@ -24,6 +27,7 @@ struct MatPair {
     // the products that open the model's expressions, rounded as it rounds them:
     // 2 Yeff, 8 Geff, 4/3 Yeff, -2 sqrt(5/6) betaeff
     double Y2, G8, Y43, b56;
+    int fast;   // Y2 and G8 in [2^-100, 2^100]: pair_contact_fast may be used
 };
 
 struct ContactOut {
@@ -181,6 +185,145 @@ __device__ __forceinline__ void pair_contact(const MatPair &M, double delx, doub
         out.T[1] = T1;
         out.T[2] = T2;
     }
+}
+
+// pair_contact<false> with the branch-free quotients and roots of
+// gb2_fastmath.cuh: the same operations on the same operands, so the same
+// bits, when every operand is in their range.  Returns false when one is not
+// (out and shear are then meaningless, and the caller evaluates the pair with
+// pair_contact).
+__device__ __forceinline__ bool pair_contact_fast(const MatPair &M, double delx, double dely, double delz, double rsq,
+                                                  double radi, double radj, const double vi[3], const double vj[3],
+                                                  const double wi[3], const double wj[3], double mi, double mj,
+                                                  double shear[3], bool update_history, double dt, bool rolling,
+                                                  bool tdamp, ContactOut &out)
+{
+    const double radsum = radi + radj, msum = mi + mj;
+    double rinv;
+    const double r = fast_sqrt(rsq, rinv);
+    bool ok = (M.fast != 0) & fast_range(rsq) & fast_divisor(r) & fast_range(radsum) & fast_divisor(radsum) &
+              fast_range(msum) & fast_divisor(msum);
+    rinv = fast_rcp_from(r, rinv);
+    const double enx = delx * rinv;
+    const double eny = dely * rinv;
+    const double enz = delz * rinv;
+    const double meff = fast_div(mi * mj, msum);
+
+    // ---- surface model (sphere kinematics)
+    const double vr1 = vi[0] - vj[0];
+    const double vr2 = vi[1] - vj[1];
+    const double vr3 = vi[2] - vj[2];
+    const double vn = vr1 * enx + vr2 * eny + vr3 * enz;
+    const double vn1 = vn * enx;
+    const double vn2 = vn * eny;
+    const double vn3 = vn * enz;
+    const double vt1 = vr1 - vn1;
+    const double vt2 = vr2 - vn2;
+    const double vt3 = vr3 - vn3;
+    const double deltan = radsum - r;
+    const double cri = radi - 0.5 * deltan;
+    const double crj = radj - 0.5 * deltan;
+    const double wr1 = (cri * wi[0] + crj * wj[0]) * rinv;
+    const double wr2 = (cri * wi[1] + crj * wj[1]) * rinv;
+    const double wr3 = (cri * wi[2] + crj * wj[2]) * rinv;
+    const double vtr1 = vt1 - (delz * wr2 - dely * wr3);
+    const double vtr2 = vt2 - (delx * wr3 - delz * wr1);
+    const double vtr3 = vt3 - (dely * wr1 - delx * wr2);
+
+    // ---- normal model (Hertz)
+    const double reff = fast_div(radi * radj, radsum);
+    const double hr = reff * deltan;
+    const double sqrtval = fast_sqrt(hr);
+    const double Sn = M.Y2 * sqrtval;
+    const double St = M.G8 * sqrtval;
+    const double kn = M.Y43 * sqrtval;
+    const double kt = St;
+    const double dn = Sn * meff, dtg = St * meff;
+    ok = ok & fast_range(meff) & fast_range(hr);   // and so dn and dtg are in [2^-400, 2^400]
+    const double gamman = M.b56 * fast_sqrt(dn);
+    const double gammat = tdamp ? M.b56 * fast_sqrt(dtg) : 0.0;
+    const double Fn_damping = -gamman * vn;
+    const double Fn_contact = kn * deltan;
+    const double Fn = Fn_damping + Fn_contact;
+    double F0 = 0.0, F1 = 0.0, F2 = 0.0;
+    F0 += Fn * enx;
+    F1 += Fn * eny;
+    F2 += Fn * enz;
+
+    // ---- tangential model (history)
+    if (update_history) {
+        shear[0] += vtr1 * dt;
+        shear[1] += vtr2 * dt;
+        shear[2] += vtr3 * dt;
+        const double rsht = shear[0] * enx + shear[1] * eny + shear[2] * enz;
+        shear[0] -= rsht * enx;
+        shear[1] -= rsht * eny;
+        shear[2] -= rsht * enz;
+    }
+    const double sq = shear[0] * shear[0] + shear[1] * shear[1] + shear[2] * shear[2];
+    ok = ok & fast_range0(sq);
+    const double shrmag = sq == 0.0 ? 0.0 : fast_sqrt(sq);
+    double Ft1 = -(kt * shear[0]);
+    double Ft2 = -(kt * shear[1]);
+    double Ft3 = -(kt * shear[2]);
+    const double Ft_shear = kt * shrmag;
+    const double Ft_friction = M.mu * fabs(Fn);
+    if (Ft_shear > Ft_friction) {
+        ok = ok & fast_range(Ft_shear) & fast_divisor(Ft_shear) & fast_range0(Ft_friction);
+        const double ratio = fast_div(Ft_friction, Ft_shear);
+        Ft1 *= ratio;
+        Ft2 *= ratio;
+        Ft3 *= ratio;
+        if (update_history) {
+            ok = ok & fast_range(fabs(Ft1)) & fast_range(fabs(Ft2)) & fast_range(fabs(Ft3)) & fast_divisor(kt);
+            const double ktinv = fast_rcp(kt);
+            shear[0] = fast_quot(-Ft1, kt, ktinv);
+            shear[1] = fast_quot(-Ft2, kt, ktinv);
+            shear[2] = fast_quot(-Ft3, kt, ktinv);
+        }
+    } else {
+        Ft1 -= (gammat * vtr1);
+        Ft2 -= (gammat * vtr2);
+        Ft3 -= (gammat * vtr3);
+    }
+    const double tor1 = eny * Ft3 - enz * Ft2;
+    const double tor2 = enz * Ft1 - enx * Ft3;
+    const double tor3 = enx * Ft2 - eny * Ft1;
+    double T0 = 0.0, T1 = 0.0, T2 = 0.0;
+    F0 += Ft1;
+    F1 += Ft2;
+    F2 += Ft3;
+    T0 += -cri * tor1;
+    T1 += -cri * tor2;
+    T2 += -cri * tor3;
+
+    // ---- rolling model (CDT, torsion torque off)
+    if (rolling) {
+        const double wrr0 = wi[0] - wj[0];
+        const double wrr1 = wi[1] - wj[1];
+        const double wrr2 = wi[2] - wj[2];
+        const double wsq = wrr0 * wrr0 + wrr1 * wrr1 + wrr2 * wrr2;
+        const double wrmag = fast_sqrt(wsq);
+        const double num = M.mur * kn * deltan * reff;
+        ok = ok & ((wsq == 0.0) | (fast_range(wsq) & fast_divisor(wrmag) & fast_range0(num)));
+        const double sc = fast_div(num, wrmag);
+        double rt0 = sc * wrr0;
+        double rt1 = sc * wrr1;
+        double rt2 = sc * wrr2;
+        const double d = rt0 * enx + rt1 * eny + rt2 * enz;
+        const double rn0 = enx * d, rn1 = eny * d, rn2 = enz * d;
+        const bool rolls = wsq > 0.;
+        T0 -= rolls ? rt0 - rn0 : 0.;
+        T1 -= rolls ? rt1 - rn1 : 0.;
+        T2 -= rolls ? rt2 - rn2 : 0.;
+    }
+    out.F[0] = F0;
+    out.F[1] = F1;
+    out.F[2] = F2;
+    out.T[0] = T0;
+    out.T[1] = T1;
+    out.T[2] = T2;
+    return ok;
 }
 
 struct ContactOutF {

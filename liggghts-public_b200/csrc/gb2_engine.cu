@@ -1467,6 +1467,7 @@ int gb2_set_materials(gb2_ctx *c, const double *youngs, const double *poisson, c
             m.G8 = 8. * m.Geff;
             m.Y43 = 4. / 3. * m.Yeff;
             m.b56 = -2. * GB2_SQRT_FIVE_OVER_SIX * m.betaeff;
+            m.fast = m.Y2 >= 0x1p-100 && m.Y2 <= 0x1p100 && m.G8 >= 0x1p-100 && m.G8 <= 0x1p100;
         }
     if (c->dmat.alloc((kMaxTypes + 1) * (kMaxTypes + 1))) return set_err(c, GB2_ERR_CUDA, "alloc");
     CK(cudaMemcpyAsync(c->dmat.p, c->hmat, sizeof c->hmat, cudaMemcpyHostToDevice, c->st));

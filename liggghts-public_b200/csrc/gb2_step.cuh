@@ -113,8 +113,21 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
         const dbl4 h = ldg4(&D.hist[s * cap + hrow]);
         double sh[3] = {sgn * h.x, sgn * h.y, sgn * h.z};   // exact: multiplying by +-1 only flips the sign
         ContactOut o;
-        pair_contact<false>(M, delx, dely, delz, rsq, pkk.w, po.w, vk, vo, wk, wo, vk4.w, vo4.w, sh, upd, D.dt,
-                            ROLLING, D.tdamp != 0, o);
+        if (!pair_contact_fast(M, delx, dely, delz, rsq, pkk.w, po.w, vk, vo, wk, wo, vk4.w, vo4.w, sh, upd, D.dt,
+                               ROLLING, D.tdamp != 0, o)) {
+            // an operand outside the fast arithmetic's range: read again, so that
+            // this rare path keeps nothing alive through the other
+            const dbl4 p1 = D.pos[kk], p2 = D.pos[other], v1 = D.vel[kk], v2 = D.vel[other], w1 = D.omg[kk],
+                       w2 = D.omg[other], h1 = D.hist[s * cap + hrow];
+            const double dx = p1.x - p2.x, dy = p1.y - p2.y, dz = p1.z - p2.z;
+            const double va[3] = {v1.x, v1.y, v1.z}, vb[3] = {v2.x, v2.y, v2.z};
+            const double wa[3] = {w1.x, w1.y, w1.z}, wb[3] = {w2.x, w2.y, w2.z};
+            sh[0] = sgn * h1.x;
+            sh[1] = sgn * h1.y;
+            sh[2] = sgn * h1.z;
+            pair_contact<false>(M, dx, dy, dz, dx * dx + dy * dy + dz * dz, p1.w, p2.w, va, vb, wa, wb, v1.w, v2.w, sh,
+                                upd, D.dt, ROLLING, D.tdamp != 0, o);
+        }
         if (own && upd) D.hist_out[e] = dbl4{(double)sh[0], (double)sh[1], (double)sh[2], 0.0};
         for (int c = 0; c < 3; c++) {
             res[c] = o.F[c];
