@@ -8,55 +8,6 @@
 #include "gb2_device.cuh"
 
 namespace gb2 {
-// An atom with more than 64 reverse or own entries, evaluated serially in
-// the reference order (rare; kept out of line so the hot loop stays small).
-template <bool ROLLING>
-__device__ __forceinline__ void serial_atom(const Dev &D, int k, const dbl4 &pk, const dbl4 &vi4, const dbl4 &wi4, int tk,
-                                         int nr, int nn, bool upd, ContactOut &acc)
-{
-    const int cap = D.cap;
-    const double vk[3] = {vi4.x, vi4.y, vi4.z}, wk[3] = {wi4.x, wi4.y, wi4.z};
-    // more than 64 entries on one side: every entry in order on this lane
-    for (int r = 0; r < nr; r++) {
-        const int i = __ldg(&D.rev[r * cap + k]);
-        const dbl4 pi = ldg4(&D.pos[i]);
-        const double delx = pk.x - pi.x;
-        const double dely = pk.y - pi.y;
-        const double delz = pk.z - pi.z;
-        const double rsq = delx * delx + dely * dely + delz * delz;
-        const double radsum = pk.w + pi.w;
-        if (!(rsq < radsum * radsum)) continue;
-        const int s = D.revs[r * cap + k];
-        const dbl4 v4 = ldg4(&D.vel[i]), w4 = ldg4(&D.omg[i]);
-        const double vi[3] = {v4.x, v4.y, v4.z}, wi[3] = {w4.x, w4.y, w4.z};
-        const dbl4 h = ldg4(&D.hist[s * cap + i]);
-        double sh[3] = {-h.x, -h.y, -h.z};
-        pair_contact(mat(D, D.type[i], tk), delx, dely, delz, rsq, pk.w, pi.w, vk, vi, wk, wi, vi4.w, v4.w, sh,
-                     upd, D.dt, ROLLING, D.tdamp != 0, acc);
-    }
-    for (int s = 0; s < nn; s++) {
-        const int e = s * cap + k;
-        const int j = __ldg(&D.nbr[e]);
-        const dbl4 pj = ldg4(&D.pos[j]);
-        const double delx = pk.x - pj.x;
-        const double dely = pk.y - pj.y;
-        const double delz = pk.z - pj.z;
-        const double rsq = delx * delx + dely * dely + delz * delz;
-        const double radsum = pk.w + pj.w;
-        const dbl4 h = ldg4(&D.hist[e]);
-        double sh[3] = {h.x, h.y, h.z};
-        if (rsq < radsum * radsum) {
-            const dbl4 v4 = ldg4(&D.vel[j]), w4 = ldg4(&D.omg[j]);
-            const double vj[3] = {v4.x, v4.y, v4.z}, wj[3] = {w4.x, w4.y, w4.z};
-            const int fl = D.flag[e];
-            if ((fl | 5) != fl) D.flag[e] = fl | 5;
-            pair_contact(mat(D, tk, D.type[j]), delx, dely, delz, rsq, pk.w, pj.w, vk, vj, wk, wj, vi4.w, v4.w,
-                         sh, upd, D.dt, ROLLING, D.tdamp != 0, acc);
-        }
-        if (upd) D.hist_out[e] = dbl4{sh[0], sh[1], sh[2], 0.0};   // serial atoms write every slot
-    }
-}
-
 // Programmatic dependent launch: the pair step lets the tail kernel be
 // scheduled as soon as all of its blocks are running; the tail kernel does
 // what does not need the pair sums first and then waits for the pair step
@@ -67,6 +18,13 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 // A kernel of a step queued ahead returns at once when an earlier step has
 // asked for a neighbour rebuild (that step's successors are redone after it).
 __device__ __forceinline__ bool step_cancelled(const Dev &D) { return D.dstop && *(volatile int *)D.dstop < D.step; }
+
+// Atoms per warp of the tail kernel: lanes 0..kTailAtoms-1 own one atom
+// each, all 32 lanes share the evaluation of their mesh candidates.
+#ifndef GB2_TAIL_ATOMS
+#define GB2_TAIL_ATOMS 8
+#endif
+constexpr int kTailAtoms = GB2_TAIL_ATOMS;
 
 // One touching pair of the warp-compacted evaluation: owner kk, the other
 // atom, the half-list slot s of the pair (in kk's list when own, in other's
@@ -132,6 +90,71 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
         for (int c = 0; c < 3; c++) {
             res[c] = o.F[c];
             res[3 + c] = o.T[c];
+        }
+    }
+}
+
+// The pair sums of an atom k with more than 64 reverse or own entries, by a
+// whole warp: the entries of a side are screened 128 at a time, the touching
+// ones listed in order (list: kLongList ints of the warp's shared memory),
+// evaluated one per lane, and added in list order -- the reference's order --
+// by every lane.  Out of line, so the tail kernel's registers are its own.  What bounds it is the chain of dependent gathers, so the
+// entries of four chunks are in flight together; one lane taking the entries
+// one by one (a 3 mm sphere in a bed of 0.3 mm spheres has hundreds) set the
+// whole step's time.  FP64 in both precisions.
+constexpr int kLongList = kTailAtoms * 64;
+
+template <bool ROLLING>
+__device__ __noinline__ void long_atom(const Dev &D, int k, int nr, int nn, bool upd, int *list, ContactOut &acc)
+{
+    const unsigned FULL = 0xffffffffu;
+    const int cap = D.cap, lane = threadIdx.x & 31;
+    const dbl4 pk = ldg4(&D.pos[k]);
+    for (int c = 0; c < 3; c++) acc.F[c] = acc.T[c] = 0.0;
+    for (int side = 0; side < 2; side++) {
+        const int tot = side ? nn : nr;
+        const int *idx = side ? D.nbr : D.rev;
+        int n = 0;
+        for (int base = 0; base < tot; base += 128) {
+            int j[4];
+            dbl4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int e = base + 32 * u + lane;
+                j[u] = e < tot ? ld_stream(&idx[e * cap + k]) : k;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) q[u] = ldg4(&D.pos[j[u]]);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int e = base + 32 * u + lane;
+                const bool t = e < tot && touching(pk, q[u]);
+                if (side && upd && e < tot && !t) D.hist_out[e * cap + k] = ldg4(&D.hist[e * cap + k]);
+                const unsigned m = __ballot_sync(FULL, t);
+                if (t) list[n + __popc(m & ((1u << lane) - 1u))] = e;
+                n += __popc(m);
+            }
+            __syncwarp();
+            if (n > kLongList - 128 || base + 128 >= tot) {
+                for (int b = 0; b < n; b += 32) {
+                    double res[6] = {0., 0., 0., 0., 0., 0.};
+                    if (b + lane < n) {
+                        const int e = list[b + lane];
+                        const int s = side ? e : (int)D.revs[e * cap + k];
+                        if (side) D.flag[e * cap + k] |= 5;   // CONTACT_NORMAL_MODEL | CONTACT_TANGENTIAL_MODEL
+                        eval_item<ROLLING, false, false>(D, k, __ldg(&idx[e * cap + k]), s, side == 1, upd, res);
+                    }
+                    const int cnt = min(32, n - b);
+                    for (int t = 0; t < cnt; t++)
+#pragma unroll
+                        for (int c = 0; c < 3; c++) {
+                            acc.F[c] += __shfl_sync(FULL, res[c], t);
+                            acc.T[c] += __shfl_sync(FULL, res[3 + c], t);
+                        }
+                }
+                n = 0;
+                __syncwarp();
+            }
         }
     }
 }
@@ -337,8 +360,7 @@ __device__ __forceinline__ void atom_fix_tail(const Dev &D, int k, const dbl4 &p
 // (reverse entries in ascending owner order, then own entries in list
 // order), evaluated one per lane in rounds of 32 with results staged in
 // shared memory, and summed by each owner lane in that order.  Atoms with
-// more than 64 reverse or own entries are evaluated serially by their owner
-// lane after the rounds, in the same order.
+// more than 64 reverse or own entries are left to the tail kernel.
 template <bool ROLLING, int MINB, bool SPLIT, bool ONE>
 __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate, int integrate, int fuse_next,
                                                          int store_f)
@@ -479,13 +501,6 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     atom_fix_tail<SPLIT>(D, k, pk, vi4, wi4, hold, integrate, fuse_next, store_f, acc);
 }
 
-// Atoms per warp of the tail kernel: lanes 0..kTailAtoms-1 own one atom
-// each, all 32 lanes share the evaluation of their mesh candidates.
-#ifndef GB2_TAIL_ATOMS
-#define GB2_TAIL_ATOMS 8
-#endif
-constexpr int kTailAtoms = GB2_TAIL_ATOMS;
-
 // Second kernel of the step: the atoms listed at the last neighbour build
 // as having wall candidates or more than 64 entries on a side, kTailAtoms
 // per warp.  Launched as a programmatic dependent of k_pair_step, it starts
@@ -494,14 +509,14 @@ constexpr int kTailAtoms = GB2_TAIL_ATOMS;
 // wall's contact history, so they are evaluated first (mesh candidates
 // spread over the lanes, slot partners staged in shared memory) and their
 // forces kept as records.  After the wait, each atom is finished from the
-// pair sums k_pair_step left in tailf/tailt (an atom with more than 64
-// entries on a side evaluates its pairs here in the reference order): the
+// pair sums k_pair_step left in tailf/tailt (the pairs of an atom with more
+// than 64 entries on a side are evaluated here, before the wait): the
 // post_force fixes in definition order with the records added at their
 // fix, walls not yet done evaluated now, then final_integrate and the
 // fused next initial_integrate.  Every atom's end of step touches only that
 // atom's records, so the result is bit for bit that of one kernel.
 template <bool ROLLING, bool SPLIT>
-__global__ void __launch_bounds__(128, 4) k_pair_tail(Dev D, int shearupdate, int integrate, int fuse_next,
+__global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ Dev D, int shearupdate, int integrate, int fuse_next,
                                                       int store_f)
 {
     __shared__ int s_sp[4][kTailAtoms * 64];            // slot partners of the warp's atoms (mesh walls)
@@ -540,6 +555,19 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(Dev D, int shearupdate, in
             }
         }
         const bool serial = nr > 64 || nn > 64;
+        // long lists, also before the wait: their sums need nothing of the pair step
+        ContactOut lacc;
+        for (int c = 0; c < 3; c++) lacc.F[c] = lacc.T[c] = 0.0;
+        for (unsigned m = __ballot_sync(0xffffffffu, own && serial); m; m &= m - 1u) {
+            const int src = __ffs(m) - 1;
+            ContactOut a;
+            long_atom<ROLLING>(D, __shfl_sync(0xffffffffu, i, src), __shfl_sync(0xffffffffu, nr, src),
+                               __shfl_sync(0xffffffffu, nn, src), upd, s_sp[wid], a);
+            if (lane == src) {
+                lacc = a;
+                if (upd) D.prevmask[i] = ~0ull;   // every own slot written this step
+            }
+        }
         const double vi[3] = {vi4.x, vi4.y, vi4.z}, wi[3] = {wi4.x, wi4.y, wi4.z};
         // walls before the wait: atoms with one wall fix at work
         bool early = own && !serial && nwork == 1;
@@ -562,8 +590,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(Dev D, int shearupdate, in
         for (int c = 0; c < 3; c++) acc.F[c] = acc.T[c] = 0.0;
         if (own) {
             if (serial) {
-                serial_atom<ROLLING>(D, i, pi, vi4, wi4, ti, nr, nn, upd, acc);
-                if (upd) D.prevmask[i] = ~0ull;   // every own slot written this step
+                acc = lacc;
             } else {
                 const dbl4 F4 = D.tailf[i], T4 = D.tailt[i];
                 acc.F[0] = F4.x;
