@@ -356,10 +356,48 @@ __device__ __forceinline__ void list_append(int2 *list, int cap, int &n, bool ta
     n += __popc(m);
 }
 
+//
+// G lanes per atom: lane G a + g takes entries g, g + G, ... of atom a's lists,
+// so a ballot's lane order is still every atom's list order; the owner lane
+// is G a, and the masks come back complete in the lanes of an atom.
+template <int G>
 __device__ __forceinline__ bool screen_list(const Dev &D, int k, int nr, int nn, const dbl4 &pk,
                                             unsigned long long &mrev, unsigned long long &mown, int2 *lrev,
                                             int2 *lown, int &nlrev, int &nlown)
 {
+    if constexpr (G > 1) {
+        const unsigned FULL = 0xffffffffu;
+        const int cap = D.cap, lane = threadIdx.x & 31, g = lane % G, owner = lane - g;
+        const int nw = __reduce_max_sync(FULL, max(nr, nn));
+        nlrev = nlown = 0;
+        for (int base = 0; base < nw; base += 2 * G) {
+            const int t0 = base + g, t1 = t0 + G;
+            const int a0 = t0 < nr ? ld_stream(&D.rev[t0 * cap + k]) : 0;
+            const int a1 = t1 < nr ? ld_stream(&D.rev[t1 * cap + k]) : 0;
+            const int b0 = t0 < nn ? ld_stream(&D.nbr[t0 * cap + k]) : 0;
+            const int b1 = t1 < nn ? ld_stream(&D.nbr[t1 * cap + k]) : 0;
+            const int s0 = t0 < nr ? (int)D.revs[t0 * cap + k] : 0;
+            const int s1 = t1 < nr ? (int)D.revs[t1 * cap + k] : 0;
+            const dbl4 qa0 = ldg4(&D.pos[a0]), qa1 = ldg4(&D.pos[a1]);
+            const dbl4 qb0 = ldg4(&D.pos[b0]), qb1 = ldg4(&D.pos[b1]);
+            const bool ta0 = t0 < nr && touching(pk, qa0), ta1 = t1 < nr && touching(pk, qa1);
+            const bool tb0 = t0 < nn && touching(pk, qb0), tb1 = t1 < nn && touching(pk, qb1);
+            if (ta0) mrev |= 1ull << t0;
+            if (ta1) mrev |= 1ull << t1;
+            if (tb0) mown |= 1ull << t0;
+            if (tb1) mown |= 1ull << t1;
+            list_append(lrev, D.item_cap, nlrev, ta0, a0, owner | (s0 << 8));
+            list_append(lrev, D.item_cap, nlrev, ta1, a1, owner | (s1 << 8));
+            list_append(lown, D.item_cap, nlown, tb0, b0, owner | (t0 << 8));
+            list_append(lown, D.item_cap, nlown, tb1, b1, owner | (t1 << 8));
+        }
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            mrev |= __shfl_xor_sync(FULL, mrev, o);
+            mown |= __shfl_xor_sync(FULL, mown, o);
+        }
+        return nlrev <= D.item_cap && nlown <= D.item_cap;
+    }
     const int cap = D.cap, lane = threadIdx.x & 31;
     const int nw = __reduce_max_sync(0xffffffffu, max(nr, nn));
     nlrev = nlown = 0;

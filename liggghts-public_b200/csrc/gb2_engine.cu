@@ -162,7 +162,6 @@ struct gb2_ctx {
     bool split = false;           // GB2_PREC_SPLIT
     DBuf<flt8> kin, kin2;         // split precision: FP32 kinematics records (double-buffered like vel)
     DBuf<uint8_t> revs;
-    int minb = 0;                 // register-allocation target of the pair step kernel (blocks/SM; 0: default)
     int nsm = 148;                // SMs of the device
     int tail_per_sm = 8;          // blocks of the tail kernel per SM (kTailAtoms atoms per warp)
     int item_cap = 160;           // listed-round capacity per warp and side (grown on demand up to kItemCap)
@@ -1209,33 +1208,20 @@ int adapt_item_cap(gb2_ctx *c)
     return 0;
 }
 
-template <bool R, int MINB>
-void launch_pair_kernel(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int fuse_next, int store_f)
-{
-    const auto kernel = D.ntypes == 1 ? k_pair_step<R, MINB, false, true> : k_pair_step<R, MINB, false, false>;
-    kernel<<<nblk(c->nlocal), kBlock, pair_list_smem(c), c->st>>>(D, shearupdate, integrate, fuse_next, store_f);
-}
-
 // The pair step kernel of one time step (every atom's pair sums; the
 // whole step for atoms without wall work).
 void launch_pair(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int fuse_next, int store_f)
 {
-    if (c->split) {
-        launch_pair_split(D, nblk(c->nlocal), c->st, c->minb, shearupdate, integrate, fuse_next, store_f,
-                          pair_list_smem(c));
-        return;
-    }
-    // MINB: minimum resident 128-thread blocks per SM asked of the register
-    // allocator; 5 (96 registers, a small spill) measured fastest on the
-    // packed 1M hopper, ahead of 4 (128) and 6 (80)
-    const int mb = c->minb ? c->minb : 5;
-    if (c->P.rolling_cdt) {
-        if (mb == 5) launch_pair_kernel<true, 5>(c, D, shearupdate, integrate, fuse_next, store_f);
-        else launch_pair_kernel<true, 6>(c, D, shearupdate, integrate, fuse_next, store_f);
-    } else {
-        if (mb == 5) launch_pair_kernel<false, 5>(c, D, shearupdate, integrate, fuse_next, store_f);
-        else launch_pair_kernel<false, 6>(c, D, shearupdate, integrate, fuse_next, store_f);
-    }
+    // Two lanes per atom while one would leave SMs with fewer than ~2 blocks:
+    // the chain of list, gather and contact rounds sets the time there, and
+    // two lanes halve it (20,000-sphere pour 40.2 -> 37.6 us/step, 6,000-sphere
+    // hopper 32.1 -> 31.0).  At 40,000 spheres both take the same, at 300,000
+    // two lanes are slower (83 -> 102).  Four lanes gain nothing on two.
+    const int lanes = c->nlocal <= 200 * c->nsm ? 2 : 1;
+    if (c->split)
+        launch_pair_split(D, lanes, c->st, shearupdate, integrate, fuse_next, store_f, pair_list_smem(c));
+    else
+        launch_pair_step<false>(D, lanes, c->st, shearupdate, integrate, fuse_next, store_f, pair_list_smem(c));
 }
 
 // The tail kernel: the atoms with wall work or more than 64 entries on a side.
@@ -1375,7 +1361,6 @@ int gb2_create(const gb2_params *p, gb2_ctx **out)
     c->P = *p;
     c->split = p->precision == GB2_PREC_SPLIT;
     if (c->P.neigh_every <= 0) c->P.neigh_every = 1;
-    if (const char *mb = std::getenv("GB2_PAIR_MINB")) c->minb = std::atoi(mb);
     if (const char *tb = std::getenv("GB2_TAIL_BLOCKS")) c->tail_per_sm = std::max(1, std::atoi(tb));
     if (const char *ic = std::getenv("GB2_ITEM_CAP")) {
         c->item_cap = std::min(std::max(std::atoi(ic), 0), kItemCap);

@@ -11,27 +11,10 @@
 
 namespace gb2 {
 
-template <bool R, int MINB>
-static void launch(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                   int store_f, size_t smem)
+void launch_pair_split(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
+                       int store_f, size_t smem)
 {
-    const auto kernel = D.ntypes == 1 ? k_pair_step<R, MINB, true, true> : k_pair_step<R, MINB, true, false>;
-    kernel<<<nblocks, 128, smem, st>>>(D, shearupdate, integrate, fuse_next, store_f);
-}
-
-void launch_pair_split(const Dev &D, int nblocks, cudaStream_t st, int minb, int shearupdate, int integrate,
-                       int fuse_next, int store_f, size_t smem)
-{
-    const int mb = minb ? minb : 5;   // 5 (96 registers, no spill) measured fastest on the packed 1M hopper
-    if (D.rolling) {
-        if (mb == 5) launch<true, 5>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f, smem);
-        else if (mb == 6) launch<true, 6>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f, smem);
-        else launch<true, 8>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f, smem);
-    } else {
-        if (mb == 5) launch<false, 5>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f, smem);
-        else if (mb == 6) launch<false, 6>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f, smem);
-        else launch<false, 8>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f, smem);
-    }
+    launch_pair_step<true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
 }
 
 void launch_tail_split(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate, int fuse_next,

@@ -160,18 +160,19 @@ __device__ __noinline__ void long_atom(const Dev &D, int k, int nr, int nn, bool
 }
 
 // FP64: plain in-order sum.  Split: FP32 sum with Kahan compensation kc.
+// v: the item's column of the staged results (components 32 apart).
 template <bool SPLIT, typename Real>
 __device__ __forceinline__ void sum_item(Real *as, Real *kc, const Real *v)
 {
 #pragma unroll
     for (int c = 0; c < 6; c++) {
         if constexpr (SPLIT) {
-            const float y = v[c] - kc[c];
+            const float y = v[32 * c] - kc[c];
             const float t = as[c] + y;
             kc[c] = (t - as[c]) - y;
             as[c] = t;
         } else {
-            as[c] += v[c];
+            as[c] += v[32 * c];
         }
     }
 }
@@ -361,12 +362,12 @@ __device__ __forceinline__ void atom_fix_tail(const Dev &D, int k, const dbl4 &p
 // order), evaluated one per lane in rounds of 32 with results staged in
 // shared memory, and summed by each owner lane in that order.  Atoms with
 // more than 64 reverse or own entries are left to the tail kernel.
-template <bool ROLLING, int MINB, bool SPLIT, bool ONE>
+template <bool ROLLING, int MINB, bool SPLIT, bool ONE, int G>
 __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate, int integrate, int fuse_next,
                                                          int store_f)
 {
     using Real = typename std::conditional<SPLIT, float, double>::type;
-    __shared__ Real sres[4][32][6];
+    __shared__ Real sres[4][6][32];   // component-major: the owners' reads and the items' writes spread over the banks
     // the atom's records that only the tail needs (velocity, angular
     // velocity, position at the last rebuild) wait here, not in registers,
     // while the screening and the contact rounds run
@@ -379,9 +380,9 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     grid_dep_launch();   // the tail kernel may be scheduled once every block of this grid runs
     if (step_cancelled(D)) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int wbase = blockIdx.x * blockDim.x + wid * 32;
-    const bool valid = k < D.nlocal;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) / G;   // G lanes per atom, the first owns it
+    const int wbase = (blockIdx.x * blockDim.x + wid * 32) / G;
+    const bool valid = k < D.nlocal, owns = valid && (G == 1 || lane % G == 0);
     const int cap = D.cap;
     const bool upd = shearupdate != 0;
     dbl4 pk;
@@ -392,9 +393,11 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     if (valid) {
         // the atom's own records, including those only the tail needs, are
         // requested first so their latency overlaps the screening
-        stage4(&stail[0][threadIdx.x], &D.vel[k]);
-        stage4(&stail[1][threadIdx.x], &D.omg[k]);
-        if (fuse_next) stage4(&stail[2][threadIdx.x], &D.xhold[k]);
+        if (owns) {
+            stage4(&stail[0][threadIdx.x], &D.vel[k]);
+            stage4(&stail[1][threadIdx.x], &D.omg[k]);
+            if (fuse_next) stage4(&stail[2][threadIdx.x], &D.xhold[k]);
+        }
         pk = D.pos[k];
         nr = D.rnum[k];
         nn = D.nnum[k];
@@ -406,8 +409,8 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     // entries (all lanes take part in the list ballots)
     int nlrev = 0, nlown = 0;
     int2 *lrev = reinterpret_cast<int2 *>(pair_dyn) + (size_t)wid * 2 * D.item_cap, *lown = lrev + D.item_cap;
-    const bool listed = screen_list(D, k, (valid && !serial) ? nr : 0, (valid && !serial) ? nn : 0, pk, mrev, mown,
-                                    lrev, lown, nlrev, nlown);
+    const bool listed = screen_list<G>(D, k, (valid && !serial) ? nr : 0, (valid && !serial) ? nn : 0, pk, mrev, mown,
+                                       lrev, lown, nlrev, nlown);
     if (!listed && lane == 0 && D.item_cap > 0) atomicAdd(&D.need[4], 1);   // lists too short: counted for the host
     // FP64 path: plain in-order sums (bit-exact).  Split path: FP32 sums of
     // the FP32 pair contributions with Kahan compensation kc.
@@ -415,43 +418,43 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
 #pragma unroll
     for (int c = 0; c < 6; c++) as[c] = kc[c] = Real(0);
     if (listed) {
-        // rounds over the listed items, rev list first: lane t evaluates item
-        // base + t; the lanes holding one owner's items find each other with
-        // a match, the first of them publishes the group to the owner, and
-        // the owner adds its items in list order
+        // rounds over the listed items, the rev list followed by the own list
+        // (a round may hold both): lane t evaluates item base + t; the lanes
+        // holding one owner's items find each other with a match, the first
+        // of them publishes the group to the owner, and the owner adds its
+        // items in list order
         sgrp[wid][lane] = ~0ull;
         __syncwarp();
+        const int tot = nlrev + nlown;
         int round = 0;
-        for (int li = 0; li < 2; li++) {
-            const int tot = li ? nlown : nlrev;
-            for (int base = 0; base < tot; base += 32, round++) {
-                const int w = base + lane;
-                int L = -1 - lane;   // lanes without an item match nobody
-                if (w < tot) {
-                    const int2 item = (li ? lown : lrev)[w];
-                    L = item.y & 31;
-                    Real res[6];
-                    eval_item<ROLLING, SPLIT, ONE>(D, wbase + L, item.x, item.y >> 8, li == 1, upd, res);
+        for (int base = 0; base < tot; base += 32, round++) {
+            const int w = base + lane;
+            int L = -1 - lane;   // lanes without an item match nobody
+            if (w < tot) {
+                const bool own = w >= nlrev;
+                const int2 item = own ? lown[w - nlrev] : lrev[w];
+                L = item.y & 31;
+                Real res[6];
+                eval_item<ROLLING, SPLIT, ONE>(D, wbase + L / G, item.x, item.y >> 8, own, upd, res);
 #pragma unroll
-                    for (int c = 0; c < 6; c++) sres[wid][lane][c] = res[c];
-                }
-                const unsigned grp = __match_any_sync(0xffffffffu, L);
-                if (w < tot && (grp & ((1u << lane) - 1u)) == 0u)
-                    sgrp[wid][L] = ((unsigned long long)(unsigned)round << 32) | grp;
-                __syncwarp();
-                const unsigned long long g = sgrp[wid][lane];
-                unsigned mine = (unsigned)(g >> 32) == (unsigned)round ? (unsigned)g : 0u;
-                while (mine) {
-                    const int q = __ffs(mine) - 1;
-                    mine &= mine - 1u;
-                    sum_item<SPLIT>(as, kc, &sres[wid][q][0]);
-                }
-                __syncwarp();
+                for (int c = 0; c < 6; c++) sres[wid][c][lane] = res[c];
             }
+            const unsigned grp = __match_any_sync(0xffffffffu, L);
+            if (w < tot && (grp & ((1u << lane) - 1u)) == 0u)
+                sgrp[wid][L] = ((unsigned long long)(unsigned)round << 32) | grp;
+            __syncwarp();
+            const unsigned long long g = sgrp[wid][lane];
+            unsigned mine = (unsigned)(g >> 32) == (unsigned)round ? (unsigned)g : 0u;
+            while (mine) {
+                const int q = __ffs(mine) - 1;
+                mine &= mine - 1u;
+                sum_item<SPLIT>(as, kc, &sres[wid][0][q]);
+            }
+            __syncwarp();
         }
     } else {   // a list outgrew its capacity: enumerate the bitmasks
         const int crev = __popcll(mrev);
-        const WarpItems it = warp_items_cnt(crev + __popcll(mown));
+        const WarpItems it = warp_items_cnt(owns ? crev + __popcll(mown) : 0);
         for (int base = 0; base < it.total; base += 32) {
             const int w = base + lane;
             const int L = item_owner(w, it.excl);
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
             const unsigned long long mrL = shfl64(mrev, L);
             const unsigned long long moL = shfl64(mown, L);
             if (w < it.total) {
-                const int kk = wbase + L;
+                const int kk = wbase + L / G;
                 const int q = w - exL;
                 const int qr = __popcll(mrL);
                 int other, s;
@@ -477,17 +480,17 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
                 Real res[6];
                 eval_item<ROLLING, SPLIT, ONE>(D, kk, other, s, own, upd, res);
 #pragma unroll
-                for (int c = 0; c < 6; c++) sres[wid][lane][c] = res[c];
+                for (int c = 0; c < 6; c++) sres[wid][c][lane] = res[c];
             }
             __syncwarp();
             const int lo = max(it.excl, base), hi = min(it.excl + it.cnt, base + 32);
-            for (int q = lo; q < hi; q++) sum_item<SPLIT>(as, kc, &sres[wid][q - base][0]);
+            for (int q = lo; q < hi; q++) sum_item<SPLIT>(as, kc, &sres[wid][0][q - base]);
             __syncwarp();
         }
     }
     ContactOut acc;
     pair_total<SPLIT>(as, kc, acc);
-    if (!valid) return;
+    if (!owns) return;
     cp_async_wait();
     if (!serial) atom_hist_tail(D, k, prevm, mown, upd);
     if (tail) {   // finished by k_pair_tail from these pair sums
@@ -632,6 +635,32 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ De
         if (own) atom_store_integrate<SPLIT>(D, i, pi, vi4, wi4, hold, integrate, fuse_next, store_f, acc);
     }
     grid_dep_wait();
+}
+
+// Host side: the pair step with one or two lanes per atom.  Registers: 5
+// blocks per SM (96) for one lane, where the chip is full; 4 (128, no spill)
+// for two, where it is not.
+template <bool ROLLING, bool SPLIT, bool ONE>
+inline void launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
+                            int store_f, size_t smem)
+{
+    const auto kernel = lanes == 1 ? k_pair_step<ROLLING, 5, SPLIT, ONE, 1> : k_pair_step<ROLLING, 4, SPLIT, ONE, 2>;
+    const int nblocks = (int)(((long)D.nlocal * lanes + 127) / 128);
+    kernel<<<nblocks, 128, smem, st>>>(D, shearupdate, integrate, fuse_next, store_f);
+}
+
+template <bool SPLIT>
+inline void launch_pair_step(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
+                             int store_f, size_t smem)
+{
+    if (D.rolling && D.ntypes == 1)
+        launch_pair_one<true, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    else if (D.rolling)
+        launch_pair_one<true, SPLIT, false>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    else if (D.ntypes == 1)
+        launch_pair_one<false, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    else
+        launch_pair_one<false, SPLIT, false>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
 }
 
 // Host side: the tail kernel launched as a programmatic dependent of the
