@@ -170,10 +170,10 @@ struct gb2_ctx {
     bool fused_pending = false;   // the previous pass B already ran this step's initial_integrate
     // steps queued ahead of the rebuild decision (see gb2_run)
     bool queue_ok = true;         // GB2_QUEUE_DEPTH=0 turns it off
-    int queue_depth = 4;
+    int queue_depth = 6;
     bool queue_active = false;
     DBuf<int> dstop;
-    int *h_stop = nullptr;        // pinned ring of stop words read back per queued step
+    int *h_stop = nullptr;        // pinned: [0] set by the device with dstop, [1] dstop read back
     cudaEvent_t qev[16] = {};
     DBuf<int> type, tag;
     int maxn = 16, maxr = 16, maxp = 16;
@@ -183,7 +183,7 @@ struct gb2_ctx {
     DBuf<dbl4> hist, hist2;
     DBuf<double> phist;
     DBuf<unsigned long long> prevmask;
-    DBuf<int> gsrc;
+    DBuf<int> gsrc, ghead, gnext;
     DBuf<dbl4> gshift;
     // bins
     double bboxlo[3], bboxhi[3], bininv[3], binsize[3];
@@ -409,6 +409,9 @@ Dev make_dev(gb2_ctx *c)
     D.phist = c->phist.p;
     D.gsrc = c->gsrc.p;
     D.gshift = c->gshift.p;
+    D.ghead = c->nghost > 0 ? c->ghead.p : nullptr;
+    D.gnext = c->gnext.p;
+    D.hstop = c->h_stop;
     for (int d = 0; d < 3; d++) {
         D.bboxlo[d] = c->bboxlo[d];
         D.bboxhi[d] = c->bboxhi[d];
@@ -574,6 +577,7 @@ int ensure_nmax(gb2_ctx *c, int need)
     CK(c->tag.grow_keep(nm, keep, c->st));
     CK(c->gsrc.grow_keep(nm, (size_t)c->nghost, c->st));
     CK(c->gshift.grow_keep(nm, (size_t)c->nghost, c->st));
+    CK(c->gnext.grow_keep(nm, (size_t)c->nghost, c->st));
     c->nmax = nm;
     return 0;
 }
@@ -970,6 +974,10 @@ int do_borders(gb2_ctx *c)
     // Comm::setup (src/comm.cpp:670-695), one proc, periodic dims only
     c->nghost = 0;
     const double cg = c->cutneighmax / 2. + c->P.skin / 2.;
+    if (c->P.periodic[0] || c->P.periodic[1] || c->P.periodic[2]) {   // no atom has a ghost yet
+        CK(c->ghead.alloc(std::max(c->cap, 1)));
+        CK(cudaMemsetAsync(c->ghead.p, 0xff, sizeof(int) * c->cap, c->st));
+    }
     for (int dim = 0; dim < 3; dim++) {
         if (!c->P.periodic[dim]) continue;
         const int nlast = c->nlocal + c->nghost;   // both swaps of a dim scan the same range
@@ -996,6 +1004,7 @@ int do_borders(gb2_ctx *c)
             const int first = c->nlocal + c->nghost;
             if (ensure_nmax(c, first + ns)) return GB2_ERR_CUDA;
             D = make_dev(c);
+            D.ghead = c->ghead.p;   // being filled (make_dev gives it once there are ghosts)
             if (ns > 0) {
                 k_border_fill<<<nblk(ns), kBlock, 0, c->st>>>(D, c->sel.p, ns, first, dim, shift);
                 CKL();
@@ -1382,7 +1391,7 @@ int gb2_create(const gb2_params *p, gb2_ctx **out)
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep_all);
         }
     }
-    // one arena slot holds h_pinned (ints 0..31) and the stop-word ring h_stop (ints 32..47)
+    // one arena slot holds h_pinned (ints 0..31) and the stop words h_stop (ints 32..33)
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
         pinned_slot_get(&c->h_pinned) != 0 || c->dstatus.alloc(1) != cudaSuccess ||
         c->ddflag.alloc(2) != cudaSuccess || c->dneed.alloc(5) != cudaSuccess || c->dstop.alloc(1) != cudaSuccess ||
@@ -2179,7 +2188,7 @@ static int one_step(gb2_ctx *c, bool last, int mode)
         if (adapt_item_cap(c)) return GB2_ERR_CUDA;
         if (prof_end(c, &e)) return GB2_ERR_CUDA;
         c->nsteps_rebuild++;
-    } else if (c->nghost > 0) {
+    } else if (c->nghost > 0 && !ghosts_prev) {   // else the previous step moved the ghosts
         Dev D = make_dev(c);
         if (prof_begin(c, PROF_FORWARD, &e)) return GB2_ERR_CUDA;
         k_forward_comm<<<nblk(c->nghost), kBlock, 0, c->st>>>(D);
@@ -2216,11 +2225,13 @@ int gb2_run(gb2_ctx *c, int nsteps)
     // it can only come from the displacement test (neigh_modify every 1
     // delay 0 check yes, no moving mesh): each queued step's kernels return
     // at once if an earlier step's tail found a displacement beyond skin/2
-    // (device word dstop = lowest such step).  The host confirms steps in
-    // order from per-step copies of dstop; at the first step that asked, it
-    // undoes the queued successors, rebuilds and continues.  Device results
-    // are those of the one-step-at-a-time loop; the GPU no longer idles
-    // while the host reads the flag every step.
+    // (device word dstop = lowest such step; the kernel that finds it also
+    // sets the page-locked word h_stop).  The host waits for an event on every
+    // second step and looks at that word -- a copy of dstop per step cost
+    // 3 us of host time and a 5 us gap between the steps' kernels.  Once it is
+    // set, the host reads dstop behind everything queued, undoes the steps
+    // after it, rebuilds and continues.  Device results are those of the
+    // one-step-at-a-time loop; the GPU does not idle while the host decides.
     bool queueable = c->queue_ok && c->P.neigh_check && c->P.neigh_every == 1 && c->P.neigh_delay == 0;
     for (int k = 0; k < c->nfix; k++)
         if (c->fix[k].mesh && c->fix[k].mesh->moving) queueable = false;
@@ -2233,17 +2244,22 @@ int gb2_run(gb2_ctx *c, int nsteps)
             continue;
         }
         // the step just run (not queued) may have asked for a rebuild of the next
-        k_queue_start<<<1, 1, 0, c->st>>>(c->dstop.p, c->ddflag.p, (int)c->ntimestep);
+        *(volatile int *)c->h_stop = 0;   // nothing is in flight that could set it
+        const long base_step = c->ntimestep;
+        k_queue_start<<<1, 1, 0, c->st>>>(c->dstop.p, c->ddflag.p, (int)base_step, c->h_stop);
         CKL();
         c->queue_active = true;
         struct Queued {
-            long ntimestep;
-            bool last;
+            bool last, event;
             size_t nev;
         };
         Queued q[16];
         int head = s, launched = s;
         bool stop = false;
+        const auto fail = [&](int rc) {
+            c->queue_active = false;
+            return rc;
+        };
         for (;;) {
             // an insertion step is never queued (it rebuilds unconditionally)
             while (launched < nsteps && launched - head < c->queue_depth &&
@@ -2252,28 +2268,32 @@ int gb2_run(gb2_ctx *c, int nsteps)
                 Q.last = launched == nsteps - 1;
                 Q.nev = c->ev_pending.size();
                 int rc = one_step(c, Q.last, 2);
-                if (rc) {
-                    c->queue_active = false;
-                    return rc;
-                }
-                Q.ntimestep = c->ntimestep;
-                cudaEvent_t &ev = c->qev[launched % 16];
-                if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-                CK(cudaMemcpyAsync(&c->h_stop[launched % 16], c->dstop.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-                CK(cudaEventRecord(ev, c->st));
+                if (rc) return fail(rc);
                 launched++;
+                // every second step, and the last one that is queued
+                Q.event = (launched - s) % 2 == 0 || launched == nsteps || ins_due(c, c->ntimestep + 1) ||
+                          c->queue_depth == 1;
+                if (Q.event) {
+                    cudaEvent_t &ev = c->qev[(launched - 1) % 16];
+                    if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
+                        return fail(GB2_ERR_CUDA);
+                    if (cudaEventRecord(ev, c->st) != cudaSuccess) return fail(GB2_ERR_CUDA);
+                }
             }
             if (head == launched) break;
-            CK(cudaEventSynchronize(c->qev[head % 16]));
-            const int v = c->h_stop[head % 16];
-            if (v == 0x7f7f7f7f || (long)v > q[head % 16].ntimestep) {
-                head++;
+            int last = head;   // the next step with an event
+            while (!q[last % 16].event) last++;
+            if (cudaEventSynchronize(c->qev[last % 16]) != cudaSuccess) return fail(GB2_ERR_CUDA);
+            if (*(volatile int *)c->h_stop == 0) {
+                head = last + 1;
                 continue;
             }
-            // step v asked for a rebuild of step v + 1: v is `head`, or the step
-            // run just before the queue (then `head` itself did nothing); the
-            // queued steps after v did nothing
-            const int first = (long)v < q[head % 16].ntimestep ? head : head + 1;
+            // a step v asked for a rebuild of step v + 1 (v may be the step run
+            // just before the queue): the queued steps after v did nothing
+            if (cudaMemcpyAsync(&c->h_stop[1], c->dstop.p, sizeof(int), cudaMemcpyDeviceToHost, c->st) != cudaSuccess ||
+                cudaStreamSynchronize(c->st) != cudaSuccess)
+                return fail(GB2_ERR_CUDA);
+            const int first = s + (int)(c->h_stop[1] - base_step);
             for (int r = launched - 1; r >= first; r--) unqueue_step(c, q[r % 16].last, q[r % 16].nev);
             launched = first;
             stop = true;

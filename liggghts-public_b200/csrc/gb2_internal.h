@@ -20,7 +20,8 @@
 //     rnum[k], rev[r*cap+k] = owner i', revs[r*cap+k] = its slot s'
 //   contact-history partners (FixContactHistory::partner_, keyed by tag):
 //     pnum[i], ptag[s*cap+i], phist[(3s+c)*cap+i]
-//   ghosts: gsrc[g] (owned source atom), gshift[g] {dx, dy, dz, -}
+//   ghosts: gsrc[g] (owned source atom), gshift[g] {dx, dy, dz, -}, and per
+//     owned atom the chain of its ghosts (ghead, gnext)
 //   split precision: kin {vx, vy, vz, m, wx, wy, wz, -} as FP32 (32 bytes),
 //     the neighbour-side operands of the FP32 contact math
 #pragma once
@@ -146,6 +147,7 @@ struct Dev {
     // ghosts
     int *gsrc;
     dbl4 *gshift;
+    int *ghead, *gnext;      // the ghosts of an owned atom: first one (-1: none), next one; null without ghosts
     // bins
     double bboxlo[3], bboxhi[3], bininv[3], binsize[3];
     int nbin[3], mbinlo[3], mbin[3], mbins;
@@ -169,6 +171,7 @@ struct Dev {
     int *dflag;              // displacement trigger
     int *dstop;              // queued-ahead steps: lowest step whose tail asked for a rebuild (null when not queuing)
     int step;                // step number of this launch (compared with *dstop)
+    int *hstop;              // page-locked host word, set with dstop
     const dbl4 *rel;         // fix insert/stream release data [4*cap] (null without a stream):
                              // {x_ins, i_step} {v_int, r_step} {v_release, -} {omega_release, -}
     int *need;               // [5] capacity demand seen by the last overflowing kernel:

@@ -104,12 +104,13 @@ __global__ void k_unpack_atoms(const dbl4 *__restrict__ pos, const dbl4 *__restr
 }
 
 // Comm::forward_comm with AtomVecSphere::pack_comm_vel (src/comm.cpp:773):
-// ghost = owned source + accumulated periodic shift
+// ghost = owned source + accumulated periodic shift.  The first step of a run
+// only: a step whose initial_integrate was fused into the previous one finds
+// its ghosts moved by their owners.
 __global__ void k_forward_comm(Dev D)
 {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= D.nghost) return;
-    if (D.dstop && *(volatile int *)D.dstop < D.step) return;   // queued step after a rebuild request
     const int src = D.gsrc[g];
     const dbl4 s = D.gshift[g];
     const dbl4 p = D.pos[src];
@@ -288,6 +289,7 @@ __global__ void k_border_fill(Dev D, const int *sel, int nsel, int first, int di
     sh.w = 0.0;
     D.gsrc[gi] = root;
     D.gshift[gi] = sh;
+    D.gnext[gi] = atomicExch(&D.ghead[root], gi);   // the order of a chain does not affect any result
     const dbl4 p = D.pos[src];
     dbl4 q;
     q.x = p.x + (dim == 0 ? shift : 0.0);
@@ -878,7 +880,11 @@ __global__ void k_tail_list(Dev D)
 
 // Start of a queue of steps: the step just run (not queued) may already
 // have asked for a rebuild of the next one through the displacement flag.
-__global__ void k_queue_start(int *dstop, const int *dflag, int step) { *dstop = *dflag ? step : 0x7f7f7f7f; }
+__global__ void k_queue_start(int *dstop, const int *dflag, int step, volatile int *hstop)
+{
+    *dstop = *dflag ? step : 0x7f7f7f7f;
+    if (*dflag) *hstop = 1;
+}
 
 // ComputeContactAtom::compute_peratom with skin 0 (src/compute_contact_atom.cpp):
 // contact if rsq <= (radi + radj)^2; an owned atom counts its own half-list

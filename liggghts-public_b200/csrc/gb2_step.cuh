@@ -282,8 +282,23 @@ __device__ __forceinline__ void atom_store_integrate(const Dev &D, int i, const 
             const double delx = p.x - h.x, dely = p.y - h.y, delz = p.z - h.z;
             if (delx * delx + dely * dely + delz * delz > D.triggersq) {
                 *D.dflag = 1;
-                if (D.dstop) atomicMin(D.dstop, D.step);
+                if (D.dstop) {
+                    atomicMin(D.dstop, D.step);
+                    *(volatile int *)D.hstop = 1;
+                }
             }
+            // the next step's forward communication: the atom's periodic
+            // images move with it (its own kernel, which copied every ghost
+            // record again, took 4-5 us of each step)
+            if (D.ghead)
+                for (int g = D.ghead[i]; g >= 0; g = D.gnext[g]) {
+                    const dbl4 s = D.gshift[g];
+                    const int gi = D.nlocal + g;
+                    D.pos_out[gi] = dbl4{p.x + s.x, p.y + s.y, p.z + s.z, p.w};
+                    D.vel_out[gi] = vi4;
+                    D.omg_out[gi] = wi4;
+                    if constexpr (SPLIT) D.kin_out[gi] = make_kin(vi4, wi4);
+                }
         }
         D.vel_out[i] = vi4;
         D.omg_out[i] = wi4;
