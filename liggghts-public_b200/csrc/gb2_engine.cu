@@ -980,36 +980,41 @@ int do_borders(gb2_ctx *c)
     }
     for (int dim = 0; dim < 3; dim++) {
         if (!c->P.periodic[dim]) continue;
-        const int nlast = c->nlocal + c->nghost;   // both swaps of a dim scan the same range
-        for (int ineed = 0; ineed < 2; ineed++) {
-            const bool low = (ineed % 2 == 0);
-            const double prd = c->P.boxhi[dim] - c->P.boxlo[dim];
-            const double bound = low ? c->P.boxlo[dim] + cg : c->P.boxhi[dim] - cg;
-            const double shift = low ? 1 * prd : -1 * prd;
-            CK(c->bflags.alloc(std::max(nlast, 1)));
-            CK(c->sel.alloc(std::max(nlast, 1)));
-            CK(c->nsel.alloc(1));
-            Dev D = make_dev(c);
-            k_border_flags<<<nblk(nlast), kBlock, 0, c->st>>>(D, nlast, dim, low ? 1 : 0, bound, c->bflags.p);
+        // both swaps of a dim scan the same range, so both are selected before
+        // the host reads the two counts (one synchronisation per dim)
+        const int nlast = c->nlocal + c->nghost;
+        const double prd = c->P.boxhi[dim] - c->P.boxlo[dim];
+        const size_t half = (size_t)std::max(nlast, 1);
+        CK(c->bflags.alloc(2 * half));
+        CK(c->sel.alloc(2 * half));
+        CK(c->nsel.alloc(2));
+        Dev D = make_dev(c);
+        size_t bytes = 0;
+        thrust::counting_iterator<int> it(0);
+        cub::DeviceSelect::Flagged(nullptr, bytes, it, c->bflags.p, c->sel.p, c->nsel.p, nlast, c->st);
+        if (cub_tmp(c, bytes)) return GB2_ERR_CUDA;
+        for (int high = 0; high < 2; high++) {
+            const double bound = high ? c->P.boxhi[dim] - cg : c->P.boxlo[dim] + cg;
+            k_border_flags<<<nblk(nlast), kBlock, 0, c->st>>>(D, nlast, dim, high ? 0 : 1, bound,
+                                                              c->bflags.p + high * half);
             CKL();
-            size_t bytes = 0;
-            thrust::counting_iterator<int> it(0);
-            cub::DeviceSelect::Flagged(nullptr, bytes, it, c->bflags.p, c->sel.p, c->nsel.p, nlast, c->st);
-            if (cub_tmp(c, bytes)) return GB2_ERR_CUDA;
             bytes = c->cubtmp.n;
-            CK(cub::DeviceSelect::Flagged(c->cubtmp.p, bytes, it, c->bflags.p, c->sel.p, c->nsel.p, nlast, c->st));
-            CK(cudaMemcpyAsync(&c->h_pinned[2], c->nsel.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-            CK(cudaStreamSynchronize(c->st));
-            const int ns = c->h_pinned[2];
-            const int first = c->nlocal + c->nghost;
-            if (ensure_nmax(c, first + ns)) return GB2_ERR_CUDA;
-            D = make_dev(c);
-            D.ghead = c->ghead.p;   // being filled (make_dev gives it once there are ghosts)
-            if (ns > 0) {
-                k_border_fill<<<nblk(ns), kBlock, 0, c->st>>>(D, c->sel.p, ns, first, dim, shift);
+            CK(cub::DeviceSelect::Flagged(c->cubtmp.p, bytes, it, c->bflags.p + high * half, c->sel.p + high * half,
+                                          c->nsel.p + high, nlast, c->st));
+        }
+        CK(cudaMemcpyAsync(&c->h_pinned[2], c->nsel.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        const int ns[2] = {c->h_pinned[2], c->h_pinned[3]};
+        if (ensure_nmax(c, c->nlocal + c->nghost + ns[0] + ns[1])) return GB2_ERR_CUDA;
+        D = make_dev(c);
+        D.ghead = c->ghead.p;   // being filled (make_dev gives it once there are ghosts)
+        for (int high = 0; high < 2; high++) {
+            if (ns[high] > 0) {
+                k_border_fill<<<nblk(ns[high]), kBlock, 0, c->st>>>(D, c->sel.p + high * half, ns[high],
+                                                                    c->nlocal + c->nghost, dim, high ? -1 * prd : 1 * prd);
                 CKL();
             }
-            c->nghost += ns;
+            c->nghost += ns[high];
         }
     }
     return 0;
@@ -1039,36 +1044,34 @@ int do_build(gb2_ctx *c)
                                        endbit, c->st));
     bytes = c->cubtmp.n;
     CK(cub::DeviceScan::ExclusiveSum(c->cubtmp.p, bytes, c->counts.p, c->bin_start.p, c->mbins + 1, c->st));
-    for (int attempt = 0; attempt < 8; attempt++) {
-        if (clear_status(c)) return GB2_ERR_CUDA;
-        D = make_dev(c);
-        k_build_list<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
-        CKL();
-        int st;
-        if (read_status(c, &st)) return GB2_ERR_CUDA;
-        if (st & ST_LOST_ATOM) return set_err(c, GB2_ERR_LOST, "an atom is outside the binned domain");
-        if (!(st & ST_NEIGH_OVERFLOW)) break;
-        if (c->maxn >= 256) return set_err(c, GB2_ERR_CAPACITY, "more than 256 neighbours per atom");
-        c->maxn = grown_capacity(c, 0, c->maxn, 256);
-        CK(c->nbr.alloc((size_t)c->maxn * c->cap));
-        CK(c->flag.alloc((size_t)c->maxn * c->cap));
-        CK(c->hist.alloc((size_t)c->maxn * c->cap));
-        CK(c->hist2.alloc((size_t)c->maxn * c->cap));
-        if (attempt == 7) return set_err(c, GB2_ERR_CAPACITY, "neighbor list capacity could not be grown");
-    }
-    for (int attempt = 0; attempt < 8; attempt++) {
+    // the list and its reverse, checked together (an overflowing list is cut
+    // at its capacity, so the reverse fill is safe and simply done again)
+    for (int attempt = 0;; attempt++) {
         if (clear_status(c)) return GB2_ERR_CUDA;
         CK(cudaMemsetAsync(c->rnum.p, 0, sizeof(int) * c->cap, c->st));
         D = make_dev(c);
+        k_build_list<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
+        CKL();
         k_rev_fill<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
         CKL();
         int st;
         if (read_status(c, &st)) return GB2_ERR_CUDA;
-        if (!(st & ST_REV_OVERFLOW)) break;
-        c->maxr = grown_capacity(c, 2, c->maxr, 1 << 20);
-        CK(c->rev.alloc((size_t)c->maxr * c->cap));
-        CK(c->revs.alloc((size_t)c->maxr * c->cap));
-        if (attempt == 7) return set_err(c, GB2_ERR_CAPACITY, "reverse list capacity could not be grown");
+        if (st & ST_LOST_ATOM) return set_err(c, GB2_ERR_LOST, "an atom is outside the binned domain");
+        if (!(st & (ST_NEIGH_OVERFLOW | ST_REV_OVERFLOW))) break;
+        if (attempt >= 16) return set_err(c, GB2_ERR_CAPACITY, "neighbor list capacity could not be grown");
+        if (st & ST_NEIGH_OVERFLOW) {
+            if (c->maxn >= 256) return set_err(c, GB2_ERR_CAPACITY, "more than 256 neighbours per atom");
+            c->maxn = grown_capacity(c, 0, c->maxn, 256);
+            CK(c->nbr.alloc((size_t)c->maxn * c->cap));
+            CK(c->flag.alloc((size_t)c->maxn * c->cap));
+            CK(c->hist.alloc((size_t)c->maxn * c->cap));
+            CK(c->hist2.alloc((size_t)c->maxn * c->cap));
+        }
+        if (st & ST_REV_OVERFLOW) {
+            c->maxr = grown_capacity(c, 2, c->maxr, 1 << 20);
+            CK(c->rev.alloc((size_t)c->maxr * c->cap));
+            CK(c->revs.alloc((size_t)c->maxr * c->cap));
+        }
     }
     D = make_dev(c);
     k_rev_sort<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
@@ -1078,11 +1081,15 @@ int do_build(gb2_ctx *c)
     return 0;
 }
 
-int do_pre_force(gb2_ctx *c)
+//
+// checked false: nothing is read back; the caller looks at the status word
+// later and, on ST_MESHSLOT_OVERFLOW, takes the new slots back
+// (undo_pre_force) and calls again with checked true, which grows the slots.
+int do_pre_force(gb2_ctx *c, bool checked)
 {
     // FixWallGran::pre_force, FixNeighlistMesh::pre_force,
     // FixContactHistoryMesh::pre_force (rebuild steps only)
-    for (int k = 0; k < c->nfix; k++) {
+    for (int k = 0; k < c->nfix && !checked; k++) {
         HostFix &H = c->fix[k];
         if (H.kind == FIX_WALL_PLANE) {
             Dev D = make_dev(c);
@@ -1107,16 +1114,24 @@ int do_pre_force(gb2_ctx *c)
                 }
                 M.bins_valid = true;
             }
+        }
+    }
+    // (after every mesh's bins: building those clears and reads the status word)
+    for (int k = 0; k < c->nfix; k++) {
+        HostFix &H = c->fix[k];
+        if (H.kind == FIX_WALL_MESH) {
+            MeshFix &M = *H.mesh;
             // candidates into fresh buffers (old slots are still needed)
             const int old_maxt = M.maxt;
             CK(M.tcnt2.alloc(c->cap));
             M.tcnt.swap(M.tcnt2);   // the old counts are not needed by the re-paging
             for (int attempt = 0; attempt < 8; attempt++) {
                 CK(M.tlist.alloc((size_t)M.maxt * c->cap));
-                if (clear_status(c)) return GB2_ERR_CUDA;
+                if (checked && clear_status(c)) return GB2_ERR_CUDA;
                 Dev D = make_dev(c);
                 k_mesh_candidates<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D, k);
                 CKL();
+                if (!checked) break;
                 int st;
                 if (read_status(c, &st)) return GB2_ERR_CUDA;
                 if (!(st & ST_MESHSLOT_OVERFLOW)) break;
@@ -1131,11 +1146,12 @@ int do_pre_force(gb2_ctx *c)
             M.snp.swap(M.snp2);
             M.spartner.swap(M.spartner2);
             M.shist.swap(M.shist2);
-            if (clear_status(c)) return GB2_ERR_CUDA;
+            if (checked && clear_status(c)) return GB2_ERR_CUDA;
             Dev D = make_dev(c);
             // old slots now live in *2 buffers
             k_mesh_repage<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D, k, M.snp2.p, M.spartner2.p, M.shist2.p, old_maxt);
             CKL();
+            if (!checked) continue;
             int st;
             if (read_status(c, &st)) return GB2_ERR_CUDA;
             if (st & ST_MESH_INTERNAL) return set_err(c, GB2_ERR_STATE, "mesh contact history inconsistent");
@@ -1144,15 +1160,33 @@ int do_pre_force(gb2_ctx *c)
     return 0;
 }
 
+// the meshes' contact slots as they were before do_pre_force
+void undo_pre_force(gb2_ctx *c)
+{
+    for (int k = 0; k < c->nfix; k++) {
+        if (c->fix[k].kind != FIX_WALL_MESH) continue;
+        MeshFix &M = *c->fix[k].mesh;
+        M.snp.swap(M.snp2);
+        M.spartner.swap(M.spartner2);
+        M.shist.swap(M.shist2);
+    }
+}
+
 // insert: an insertion fix adds atoms on this step.  Modify::
 // list_init_pre_exchange (src/modify.cpp:1342-1367) calls the contact-history
 // fixes first, so the pair and mesh histories are packed with the last
 // build's ghost tags before the new atoms take the first ghost slots.
 int do_rebuild(gb2_ctx *c, bool pre_exchange, bool sort_now, bool insert, bool ghosts_prev)
 {
-    if (pre_exchange)
-        if (do_partners(c)) return GB2_ERR_CUDA;
+    // the partners are checked with the box test below, which does not touch
+    // them, unless an insertion comes between
+    if (insert && pre_exchange && do_partners(c)) return GB2_ERR_CUDA;
+    if (clear_status(c)) return GB2_ERR_CUDA;
     Dev D = make_dev(c);
+    if (pre_exchange && !insert) {
+        k_partners<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
+        CKL();
+    }
     for (int k = 0; k < c->nfix; k++)
         if (c->fix[k].kind == FIX_WALL_MESH) {
             k_mesh_sort_contacts<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D, k);
@@ -1162,8 +1196,8 @@ int do_rebuild(gb2_ctx *c, bool pre_exchange, bool sort_now, bool insert, bool g
         const int rci = c->stream ? do_insert_stream(c, ghosts_prev) : do_insert(c, ghosts_prev);
         if (rci) return rci;
         D = make_dev(c);
+        if (clear_status(c)) return GB2_ERR_CUDA;
     }
-    if (clear_status(c)) return GB2_ERR_CUDA;
     k_pbc<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D, c->P.boxlo[0], c->P.boxlo[1], c->P.boxlo[2], c->P.boxhi[0],
                                                   c->P.boxhi[1], c->P.boxhi[2], c->P.periodic[0], c->P.periodic[1],
                                                   c->P.periodic[2]);
@@ -1171,25 +1205,38 @@ int do_rebuild(gb2_ctx *c, bool pre_exchange, bool sort_now, bool insert, bool g
     int st;
     if (read_status(c, &st)) return GB2_ERR_CUDA;
     if (st & ST_LOST_ATOM) return set_err(c, GB2_ERR_LOST, "atom left the non-periodic box (lost atoms unsupported)");
+    if (st & ST_PARTNER_OVERFLOW)   // once more, with the capacity grown
+        if (do_partners(c)) return GB2_ERR_CUDA;
     if (sort_now)
         if (do_atom_sort(c)) return GB2_ERR_CUDA;
     if (do_borders(c)) return GB2_ERR_CUDA;
     if (do_build(c)) return c->err.empty() ? GB2_ERR_CUDA : GB2_ERR_CAPACITY;
-    {
-        const int rc = do_pre_force(c);
+    if (clear_status(c)) return GB2_ERR_CUDA;
+    for (bool checked = false;; checked = true) {
+        const int rc = do_pre_force(c, checked);
         if (rc) return (rc == GB2_ERR_UNSUPPORTED || rc == GB2_ERR_STATE) ? rc : GB2_ERR_CUDA;
+        // atoms finished by the tail kernel until the next build
+        CK(cudaMemsetAsync(c->dtailcnt.p, 0, sizeof(int), c->st));
+        if (c->nlocal > 0) {
+            Dev D3 = make_dev(c);
+            k_tail_list<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D3);
+            CKL();
+        }
+        if (checked) break;
+        // the last look at the device: the meshes' slots, and the count of
+        // short item lists for adapt_item_cap
+        CK(cudaMemcpyAsync(&c->h_pinned[6], c->dneed.p + 4, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+        if (read_status(c, &st)) return GB2_ERR_CUDA;
+        if (!(st & ST_MESHSLOT_OVERFLOW)) {
+            if (st & ST_MESH_INTERNAL) return set_err(c, GB2_ERR_STATE, "mesh contact history inconsistent");
+            break;
+        }
+        undo_pre_force(c);
     }
     if (c->split) {   // FP32 kinematics of owned atoms and the new ghosts
         const int nall = c->nlocal + c->nghost;
         Dev D2 = make_dev(c);
         if (nall > 0) k_make_kin<<<nblk(nall), kBlock, 0, c->st>>>(D2, nall);
-        CKL();
-    }
-    // atoms finished by the tail kernel until the next build
-    CK(cudaMemsetAsync(c->dtailcnt.p, 0, sizeof(int), c->st));
-    if (c->nlocal > 0) {
-        Dev D3 = make_dev(c);
-        k_tail_list<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D3);
         CKL();
     }
     return 0;
@@ -1204,11 +1251,14 @@ size_t pair_list_smem(const gb2_ctx *c) { return (size_t)4 * 2 * c->item_cap * s
 // lists grow by half, up to kItemCap, while any warp did.  Short lists keep
 // shared memory, and with it L1 for the neighbour gathers, on beds with few
 // contacts per atom.
-int adapt_item_cap(gb2_ctx *c)
+// The count is the one do_rebuild read (fresh false) or read here.
+int adapt_item_cap(gb2_ctx *c, bool fresh)
 {
     if (c->item_cap_fixed || c->item_cap >= kItemCap) return 0;
-    CK(cudaMemcpyAsync(&c->h_pinned[6], c->dneed.p + 4, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    if (fresh) {
+        CK(cudaMemcpyAsync(&c->h_pinned[6], c->dneed.p + 4, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+        CK(cudaStreamSynchronize(c->st));
+    }
     if (c->h_pinned[6] > 0) {
         c->item_cap = std::min(kItemCap, (c->item_cap * 3 / 2 + 31) / 32 * 32);
         c->item_cap_grown++;
@@ -1911,8 +1961,8 @@ int gb2_setup(gb2_ctx *c)
     int rc = do_rebuild(c, c->computeflag, c->P.sort_freq > 0, false, false);
     if (rc) return rc;
     if (do_force(c, 0, 0, 0, 1)) return GB2_ERR_CUDA;
+    if (adapt_item_cap(c, true)) return GB2_ERR_CUDA;
     CK(cudaStreamSynchronize(c->st));
-    if (adapt_item_cap(c)) return GB2_ERR_CUDA;
     if (c->ins) {   // FixInsert::setup: region volume by Monte Carlo
         const std::string e = c->ins->setup();
         if (!e.empty()) return set_err(c, GB2_ERR_ARG, "fix insert/pack: %s", e.c_str());
@@ -2185,7 +2235,7 @@ static int one_step(gb2_ctx *c, bool last, int mode)
         if (prof_begin(c, PROF_REBUILD, &e)) return GB2_ERR_CUDA;
         int rc = do_rebuild(c, true, sort_now, insert_now, ghosts_prev);
         if (rc) return rc;
-        if (adapt_item_cap(c)) return GB2_ERR_CUDA;
+        if (adapt_item_cap(c, false)) return GB2_ERR_CUDA;
         if (prof_end(c, &e)) return GB2_ERR_CUDA;
         c->nsteps_rebuild++;
     } else if (c->nghost > 0 && !ghosts_prev) {   // else the previous step moved the ghosts
