@@ -2196,21 +2196,21 @@ static int one_step(gb2_ctx *c, bool last, int mode)
     for (int k = 0; k < c->nfix; k++) {
         MeshFix *M = c->fix[k].mesh;
         if (!M || !M->moving) continue;
-        if (!moving) CK(cudaMemsetAsync(c->ddflag.p + 1, 0, sizeof(int), c->st));
+        if (!moving && mode != 2) CK(cudaMemsetAsync(c->ddflag.p + 1, 0, sizeof(int), c->st));
         moving = true;
         if (M->next_reneighbor == c->ntimestep) forced = true;   // Neighbor::decide must_check
         const int nt = (int)M->topo.tri.size();
+        const MeshMoved mm{c->ddflag.p + 1, mode == 2 ? c->dstop.p : nullptr, (int)c->ntimestep, c->h_stop};
         if (M->mover == 2) {
             const double dt = c->P.dt;
             k_mesh_translate<<<nblk(nt), kBlock, 0, c->st>>>(M->tri.p, nt, M->vnode.p, M->node_last.p,
                                                              M->mv_vel[0] * dt, M->mv_vel[1] * dt, M->mv_vel[2] * dt,
                                                              M->mv_vel[0], M->mv_vel[1], M->mv_vel[2],
-                                                             0.25 * c->P.skin * c->P.skin, c->ddflag.p + 1);
+                                                             0.25 * c->P.skin * c->P.skin, mm);
         } else {
             MeshRotate mv;
             mesh_rotation(c, *M, mv);
-            k_mesh_rotate<<<nblk(nt), kBlock, 0, c->st>>>(M->tri.p, nt, M->vnode.p, M->node_last.p, mv,
-                                                          c->ddflag.p + 1);
+            k_mesh_rotate<<<nblk(4l * nt), kBlock, 0, c->st>>>(M->tri.p, nt, M->vnode.p, M->node_last.p, mv, mm);
         }
         CKL();
     }
@@ -2272,9 +2272,9 @@ int gb2_run(gb2_ctx *c, int nsteps)
     if (!c) return GB2_ERR_ARG;
     if (!c->setup_done) return set_err(c, GB2_ERR_STATE, "gb2_setup must precede gb2_run");
     // Steps are queued up to queue_depth ahead of the rebuild decision when
-    // it can only come from the displacement test (neigh_modify every 1
-    // delay 0 check yes, no moving mesh): each queued step's kernels return
-    // at once if an earlier step's tail found a displacement beyond skin/2
+    // it can only come from a displacement test (neigh_modify every 1 delay 0
+    // check yes): each queued step's kernels return at once if an earlier
+    // step's tail, or its mesh motion, found a displacement beyond skin/2
     // (device word dstop = lowest such step; the kernel that finds it also
     // sets the page-locked word h_stop).  The host waits for an event on every
     // second step and looks at that word -- a copy of dstop per step cost
@@ -2282,12 +2282,16 @@ int gb2_run(gb2_ctx *c, int nsteps)
     // set, the host reads dstop behind everything queued, undoes the steps
     // after it, rebuilds and continues.  Device results are those of the
     // one-step-at-a-time loop; the GPU does not idle while the host decides.
-    bool queueable = c->queue_ok && c->P.neigh_check && c->P.neigh_every == 1 && c->P.neigh_delay == 0;
-    for (int k = 0; k < c->nfix; k++)
-        if (c->fix[k].mesh && c->fix[k].mesh->moving) queueable = false;
+    const bool queueable = c->queue_ok && c->P.neigh_check && c->P.neigh_every == 1 && c->P.neigh_delay == 0;
+    // a mesh that moved far on a step by itself forces the next step's rebuild
+    const auto mesh_asked = [c](long step) {
+        for (int k = 0; k < c->nfix; k++)
+            if (c->fix[k].mesh && c->fix[k].mesh->moving && c->fix[k].mesh->next_reneighbor == step) return true;
+        return false;
+    };
     int s = 0;
     while (s < nsteps) {
-        if (!queueable || !c->fused_pending || ins_due(c, c->ntimestep + 1)) {
+        if (!queueable || !c->fused_pending || ins_due(c, c->ntimestep + 1) || mesh_asked(c->ntimestep + 1)) {
             int rc = one_step(c, s == nsteps - 1, 0);
             if (rc) return rc;
             s++;

@@ -596,6 +596,28 @@ __device__ __forceinline__ void vec_quat_rotate(double *vec, const double *q)
     vec[2] = r[3];
 }
 
+// What a mover's displacement test does (a node further than skin/2 from its
+// place at the last rebuild forces a rebuild on the next step): on a step by
+// itself it sets a flag for the host; on a queued step it asks for the rebuild
+// as an atom's displacement does, and like every queued kernel it does nothing
+// once an earlier step has asked.
+struct MeshMoved {
+    int *flag;
+    int *dstop;   // null when not queued
+    int step;
+    volatile int *hstop;
+    __device__ __forceinline__ bool cancelled() const { return dstop && *(volatile int *)dstop < step; }
+    __device__ __forceinline__ void far() const
+    {
+        if (dstop) {
+            atomicMin(dstop, step);
+            *hstop = 1;
+        } else {
+            *flag = 1;
+        }
+    }
+};
+
 struct MeshRotate {
     double dQ[4];          // rotation of one step
     double origin[3];      // axis point
@@ -610,45 +632,57 @@ struct MeshRotate {
 // properties, src/surface_mesh_I.h:75-77, src/general_container_I.h:642),
 // node velocities omega x (node - origin); and MultiNodeMesh::decideRebuild's
 // displacement test against the nodes of the last rebuild (src/multi_node_mesh_I.h:791)
-__global__ void k_mesh_rotate(TriGeom *tri, int ntri, double *vnode, const double *node_last, MeshRotate mv, int *flag)
+//
+// Four lanes per triangle -- a node with its edge vector, edge normal and
+// velocity each, and the surface normal with the centre -- and every load
+// before the first store: one thread per triangle was a chain of ten
+// load-rotate-store round trips, 13.8 us for 1,632 triangles.
+__global__ void k_mesh_rotate(TriGeom *tri, int ntri, double *vnode, const double *node_last, MeshRotate mv, MeshMoved mm)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntri) return;
-    TriGeom &T = tri[t];
-    double ctr[3] = {0., 0., 0.};
-    for (int j = 0; j < 3; j++) {
-        double nd[3] = {T.node[j][0], T.node[j][1], T.node[j][2]};
+    if (mm.cancelled()) return;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x, t = g >> 2, j = g & 3;
+    const bool valid = t < ntri;
+    TriGeom &T = tri[valid ? t : 0];
+    const bool node = valid && j < 3;
+    double nd[3] = {0., 0., 0.}, ev[3] = {0., 0., 0.}, en[3] = {0., 0., 0.}, o[3] = {0., 0., 0.};
+    if (node) {
+        for (int c = 0; c < 3; c++) {
+            nd[c] = T.node[j][c];
+            ev[c] = T.edgevec[j][c];
+            en[c] = T.edgenorm[j][c];
+            o[c] = node_last[9 * t + 3 * j + c];
+        }
         if (mv.trans)
             for (int c = 0; c < 3; c++) nd[c] = nd[c] - mv.origin[c];
         vec_quat_rotate(nd, mv.dQ);
         if (mv.trans)
             for (int c = 0; c < 3; c++) nd[c] = nd[c] + mv.origin[c];
-        for (int c = 0; c < 3; c++) {
-            T.node[j][c] = nd[c];
-            ctr[c] = nd[c] + ctr[c];
-        }
-    }
-    const double sinv = 1. / 3.0;
-    for (int c = 0; c < 3; c++) T.center[c] = sinv * ctr[c];
-    for (int j = 0; j < 3; j++) {
-        vec_quat_rotate(T.edgevec[j], mv.dQ);
-        vec_quat_rotate(T.edgenorm[j], mv.dQ);
-    }
-    vec_quat_rotate(T.surfnorm, mv.dQ);
-    bool far = false;
-    for (int j = 0; j < 3; j++) {
-        const double r0 = T.node[j][0] - mv.origin[0], r1 = T.node[j][1] - mv.origin[1],
-                     r2 = T.node[j][2] - mv.origin[2];
+        vec_quat_rotate(ev, mv.dQ);
+        vec_quat_rotate(en, mv.dQ);
+        const double r0 = nd[0] - mv.origin[0], r1 = nd[1] - mv.origin[1], r2 = nd[2] - mv.origin[2];
         const double w0 = mv.omegaVec[0], w1 = mv.omegaVec[1], w2 = mv.omegaVec[2];
         double *vn = vnode + 9 * t + 3 * j;
         vn[0] = 0. + (w1 * r2 - w2 * r1);
         vn[1] = 0. + (w2 * r0 - w0 * r2);
         vn[2] = 0. + (w0 * r1 - w1 * r0);
-        const double *o = node_last + 9 * t + 3 * j;
-        const double d0 = T.node[j][0] - o[0], d1 = T.node[j][1] - o[1], d2 = T.node[j][2] - o[2];
-        if (d0 * d0 + d1 * d1 + d2 * d2 > mv.triggersq) far = true;
+        for (int c = 0; c < 3; c++) {
+            T.node[j][c] = nd[c];
+            T.edgevec[j][c] = ev[c];
+            T.edgenorm[j][c] = en[c];
+        }
+        const double d0 = nd[0] - o[0], d1 = nd[1] - o[1], d2 = nd[2] - o[2];
+        if (d0 * d0 + d1 * d1 + d2 * d2 > mv.triggersq) mm.far();
+    } else if (valid) {
+        for (int c = 0; c < 3; c++) nd[c] = T.surfnorm[c];
+        vec_quat_rotate(nd, mv.dQ);
+        for (int c = 0; c < 3; c++) T.surfnorm[c] = nd[c];
     }
-    if (far) *flag = 1;
+    double ctr[3] = {0., 0., 0.};
+    for (int q = 0; q < 3; q++)
+        for (int c = 0; c < 3; c++) ctr[c] = __shfl_sync(0xffffffffu, nd[c], (threadIdx.x & 28) + q) + ctr[c];
+    const double sinv = 1. / 3.0;
+    if (valid && j == 3)
+        for (int c = 0; c < 3; c++) T.center[c] = sinv * ctr[c];
 }
 
 // One step of MeshMoverLinear::initial_integrate (src/mesh_mover_linear.cpp:94-112)
@@ -656,8 +690,9 @@ __global__ void k_mesh_rotate(TriGeom *tri, int ntri, double *vnode, const doubl
 // src/multi_node_mesh_I.h:502-513), node velocities 0 + v, and the
 // displacement test of MultiNodeMesh::decideRebuild
 __global__ void k_mesh_translate(TriGeom *tri, int ntri, double *vnode, const double *node_last, double dx0,
-                                 double dx1, double dx2, double v0, double v1, double v2, double triggersq, int *flag)
+                                 double dx1, double dx2, double v0, double v1, double v2, double triggersq, MeshMoved mm)
 {
+    if (mm.cancelled()) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntri) return;
     TriGeom &T = tri[t];
@@ -674,7 +709,7 @@ __global__ void k_mesh_translate(TriGeom *tri, int ntri, double *vnode, const do
         if (d0 * d0 + d1 * d1 + d2 * d2 > triggersq) far = true;
     }
     for (int c = 0; c < 3; c++) T.center[c] = T.center[c] + dx[c];
-    if (far) *flag = 1;
+    if (far) mm.far();
 }
 
 // A moving mesh on a rebuild step (FixMesh::pre_force -> pbcExchangeBorders,
