@@ -205,6 +205,80 @@ __global__ void k_sq_hold(SqDev D)
     D.xhold[i] = D.x[i];
 }
 
+// bounding_sphere_radius_superquadric with n1 = n2 = n, times scale_koef 1.0001
+// (src/math_extra_liggghts_superquadric.cpp:206-233)
+__device__ double bounding_radius(double sa, double sb, double c, double n)
+{
+    if (n == 2.0 || fabs(n - 2.0) < 1e-13) return fmax(fmax(sa, sb), c) * 1.0001;
+    const double a = fmax(sa, sb), b = fmin(sa, sb);
+    const double n1 = fmax(2.1, n), n2 = n1;
+    const double alpha = pow_abs(b / a, 2.0 / (n2 - 2.0));
+    const double gamma = pow_abs(1.0 + pow_abs(alpha, n2), n1 / n2 - 1.0);
+    const double beta = pow_abs(c * c / (a * a) * gamma, 1.0 / (n1 - 2.0));
+    const double x0 = 1.0 / pow_abs(pow_abs(1.0 + pow_abs(alpha, n2), n1 / n2) + pow_abs(beta, n1), 1.0 / n1);
+    const double xt = x0 * a, yt = alpha * x0 * b, zt = beta * x0 * c;
+    return sqrt(xt * xt + yt * yt + zt * zt) * 1.0001;
+}
+
+// Particle upload: the caller's arrays staged one after another (x 3, v 3,
+// quat 4, angmom 3, shape 3, blockiness, mass, inertia 3, volume: 22 n
+// doubles), checked, then packed into the records with the bounding and
+// volume-equivalent radii (src/pair_gran_base.h:266-270).  On one host thread
+// the five powers per particle and the packing took 40 ms for 200,000.
+struct SqStage {
+    const double *x, *v, *q, *L, *sh, *blk, *m, *in3, *vol;
+    __host__ __device__ SqStage(const double *in, size_t n)
+        : x(in), v(x + 3 * n), q(v + 3 * n), L(q + 4 * n), sh(L + 3 * n), blk(sh + 3 * n), m(blk + n), in3(m + n),
+          vol(in3 + 3 * n)
+    {
+    }
+};
+
+// chk[0]: the first particle with a non-positive shape, mass or volume or a
+// blockiness below 2
+__global__ void k_sq_check(const double *__restrict__ in, int n, unsigned long long *chk)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const SqStage S(in, n);
+    if (!(S.blk[i] >= 2.0) || !(S.sh[3 * i] > 0) || !(S.sh[3 * i + 1] > 0) || !(S.sh[3 * i + 2] > 0) ||
+        !(S.m[i] > 0) || !(S.vol[i] > 0))
+        atomicMin(&chk[0], (unsigned long long)i);
+}
+
+// chk[1]: the largest bounding radius as its bits (positive numbers order as
+// their bits do)
+__global__ void k_sq_pack(SqDev D, const double *__restrict__ in, unsigned long long *chk)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= D.n) return;
+    const SqStage S(in, D.n);
+    const double *x = S.x, *v = S.v, *q = S.q, *L = S.L, *sh = S.sh, *m = S.m, *in3 = S.in3, *vol = S.vol;
+    const double s0 = sh[3 * i], s1 = sh[3 * i + 1], s2 = sh[3 * i + 2], b = S.blk[i];
+    const double rb = bounding_radius(s0, s1, s2, b);
+    atomicMax(&chk[1], (unsigned long long)__double_as_longlong(rb));
+    D.x[i] = dbl4{x[3 * i], x[3 * i + 1], x[3 * i + 2], rb};
+    D.v[i] = dbl4{v[3 * i], v[3 * i + 1], v[3 * i + 2], m[i]};
+    D.q[i] = dbl4{q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]};
+    D.L[i] = dbl4{L[3 * i], L[3 * i + 1], L[3 * i + 2], 0.0};
+    D.shape[i] = dbl4{s0, s1, s2, b};
+    D.inert[i] = dbl4{in3[3 * i], in3[3 * i + 1], in3[3 * i + 2], cbrt(0.75 * vol[i] / M_PI)};
+    D.f[i] = D.t[i] = dbl4{0.0, 0.0, 0.0, 0.0};
+}
+
+// Particle download: records to [n][k] planes, k = 3 or 4
+__global__ void k_sq_unpack(const dbl4 *__restrict__ rec, int n, int k, double *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const dbl4 r = rec[i];
+    double *o = out + (size_t)k * i;
+    o[0] = r.x;
+    o[1] = r.y;
+    o[2] = r.z;
+    if (k == 4) o[3] = r.w;
+}
+
 __global__ void k_sq_coords(SqDev D, double *xs)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -249,6 +323,8 @@ struct gb2_sq_ctx {
     Buf<int> work;
     Buf<signed char> kind;   // per slot: the work list the screen puts it on
     Buf<float4> guess;       // learned guesses of the first contacts, by list position
+    Buf<double> stage;       // particle upload and download
+    Buf<unsigned long long> chk;
     int nsm = 148;
 };
 
@@ -537,77 +613,41 @@ int gb2_sq_destroy(gb2_sq_ctx *c)
     return 0;
 }
 
-// bounding_sphere_radius_superquadric with n1 = n2 = n, times scale_koef 1.0001
-// (src/math_extra_liggghts_superquadric.cpp:206-233)
-static double host_pow_abs(double base, double e)
-{
-    base = std::fabs(base);
-    const double tol = 1e-12;
-    if (std::fabs(e) < tol || std::fabs(base - 1.0) < tol) return 1.0;
-    if (std::fabs(base) < tol) return 0.0;
-    const double nn = std::floor(std::fabs(e));
-    double r = 1.0;
-    for (int i = 0; i < (int)nn; i++) r *= base;
-    const double nd = std::fabs(e) - nn;
-    if (nd > 0.0) r *= (std::fabs(2.0 * nd - 1.0) < 2.0 * tol) ? std::sqrt(base) : std::pow(base, nd);
-    return e > 0.0 ? r : 1.0 / r;
-}
-static double bounding_radius(const double *shape, double n)
-{
-    if (n == 2.0 || std::fabs(n - 2.0) < 1e-13) return std::max(std::max(shape[0], shape[1]), shape[2]) * 1.0001;
-    const double a = std::max(shape[0], shape[1]), b = std::min(shape[0], shape[1]), c = shape[2];
-    const double n1 = std::max(2.1, n), n2 = std::max(2.1, n);
-    const double alpha = host_pow_abs(b / a, 2.0 / (n2 - 2.0));
-    const double gamma = host_pow_abs(1.0 + host_pow_abs(alpha, n2), n1 / n2 - 1.0);
-    const double beta = host_pow_abs(c * c / (a * a) * gamma, 1.0 / (n1 - 2.0));
-    const double x0 = 1.0 / host_pow_abs(host_pow_abs(1.0 + host_pow_abs(alpha, n2), n1 / n2) + host_pow_abs(beta, n1), 1.0 / n1);
-    const double xt = x0 * a, yt = alpha * x0 * b, zt = beta * x0 * c;
-    return std::sqrt(xt * xt + yt * yt + zt * zt) * 1.0001;
-}
-
 int gb2_sq_upload(gb2_sq_ctx *c, int n, const double *x, const double *v, const double *quat, const double *angmom,
                   const double *shape, const double *blockiness, const double *rmass, const double *inertia,
                   const double *volume)
 {
     if (!c || n <= 0 || !x || !v || !quat || !angmom || !shape || !blockiness || !rmass || !inertia || !volume)
         return GB2_ERR_ARG;
-    std::vector<dbl4> hx(n), hv(n), hq(n), hL(n), hs(n), hi(n);
-    double rbmax = 0;
-    for (int i = 0; i < n; i++) {
-        if (!(blockiness[i] >= 2.0) || !(shape[3 * i] > 0) || !(shape[3 * i + 1] > 0) || !(shape[3 * i + 2] > 0) ||
-            !(rmass[i] > 0) || !(volume[i] > 0))
-            return sq_err(c, GB2_ERR_ARG, "superquadric %d: shape, blockiness (>= 2), mass and volume must be positive", i);
-        const double rb = bounding_radius(&shape[3 * i], blockiness[i]);
-        rbmax = std::max(rbmax, rb);
-        hx[i] = dbl4{x[3 * i], x[3 * i + 1], x[3 * i + 2], rb};
-        hv[i] = dbl4{v[3 * i], v[3 * i + 1], v[3 * i + 2], rmass[i]};
-        hq[i] = dbl4{quat[4 * i], quat[4 * i + 1], quat[4 * i + 2], quat[4 * i + 3]};
-        hL[i] = dbl4{angmom[3 * i], angmom[3 * i + 1], angmom[3 * i + 2], 0.0};
-        hs[i] = dbl4{shape[3 * i], shape[3 * i + 1], shape[3 * i + 2], blockiness[i]};
-        // volume-equivalent radius used for the Hertz reff (src/pair_gran_base.h:266-270)
-        hi[i] = dbl4{inertia[3 * i], inertia[3 * i + 1], inertia[3 * i + 2], std::cbrt(0.75 * volume[i] / M_PI)};
+    const double *src[9] = {x, v, quat, angmom, shape, blockiness, rmass, inertia, volume};
+    const size_t len[9] = {3, 3, 4, 3, 3, 1, 1, 3, 1};
+    const size_t N = (size_t)n;
+    SQCK(c->stage.alloc(22 * N));
+    SQCK(c->chk.alloc(2));
+    size_t off = 0;
+    for (int k = 0; k < 9; k++) {
+        SQCK(cudaMemcpyAsync(c->stage.p + off, src[k], len[k] * N * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        off += len[k] * N;
     }
-    c->n = n;
-    c->rbmax = rbmax;
-    SQCK(c->x.alloc(n));
-    SQCK(c->v.alloc(n));
-    SQCK(c->q.alloc(n));
-    SQCK(c->L.alloc(n));
-    SQCK(c->w.alloc(n));
-    SQCK(c->f.alloc(n));
-    SQCK(c->t.alloc(n));
-    SQCK(c->shape.alloc(n));
-    SQCK(c->inert.alloc(n));
-    SQCK(c->xhold.alloc(n));
-    SQCK(cudaMemcpyAsync(c->x.p, hx.data(), sizeof(dbl4) * n, cudaMemcpyHostToDevice, c->st));
-    SQCK(cudaMemcpyAsync(c->v.p, hv.data(), sizeof(dbl4) * n, cudaMemcpyHostToDevice, c->st));
-    SQCK(cudaMemcpyAsync(c->q.p, hq.data(), sizeof(dbl4) * n, cudaMemcpyHostToDevice, c->st));
-    SQCK(cudaMemcpyAsync(c->L.p, hL.data(), sizeof(dbl4) * n, cudaMemcpyHostToDevice, c->st));
-    SQCK(cudaMemcpyAsync(c->shape.p, hs.data(), sizeof(dbl4) * n, cudaMemcpyHostToDevice, c->st));
-    SQCK(cudaMemcpyAsync(c->inert.p, hi.data(), sizeof(dbl4) * n, cudaMemcpyHostToDevice, c->st));
-    SQCK(cudaMemsetAsync(c->f.p, 0, sizeof(dbl4) * n, c->st));
-    SQCK(cudaMemsetAsync(c->t.p, 0, sizeof(dbl4) * n, c->st));
+    unsigned long long chk[2];
+    SQCK(cudaMemsetAsync(c->chk.p, 0xff, sizeof(unsigned long long), c->st));
+    SQCK(cudaMemsetAsync(c->chk.p + 1, 0, sizeof(unsigned long long), c->st));
+    k_sq_check<<<nb(n), kB, 0, c->st>>>(c->stage.p, n, c->chk.p);
+    SQCKL();
+    SQCK(cudaMemcpyAsync(chk, c->chk.p, sizeof chk, cudaMemcpyDeviceToHost, c->st));
     SQCK(cudaStreamSynchronize(c->st));
+    if (chk[0] < (unsigned long long)n)   // the context keeps what it held
+        return sq_err(c, GB2_ERR_ARG,
+                      "superquadric %d: shape, blockiness (>= 2), mass and volume must be positive", (int)chk[0]);
+    c->n = n;
+    for (Buf<dbl4> *b : {&c->x, &c->v, &c->q, &c->L, &c->w, &c->f, &c->t, &c->shape, &c->inert, &c->xhold})
+        SQCK(b->alloc(N));
+    SqDev D = sq_dev(c);
+    k_sq_pack<<<nb(n), kB, 0, c->st>>>(D, c->stage.p, c->chk.p);
+    SQCKL();
+    SQCK(cudaMemcpyAsync(chk, c->chk.p, sizeof chk, cudaMemcpyDeviceToHost, c->st));
+    SQCK(cudaStreamSynchronize(c->st));
+    std::memcpy(&c->rbmax, &chk[1], sizeof c->rbmax);
     c->setup_done = false;
     return 0;
 }
@@ -688,22 +728,24 @@ int gb2_sq_download(gb2_sq_ctx *c, int cap, double *x, double *v, double *quat, 
 {
     if (!c || cap < c->n) return GB2_ERR_ARG;
     const int n = c->n;
-    std::vector<dbl4> h(n);
+    if (n == 0) return 0;
+    // unpacked on the device into one block of planes, one copy per array asked for
     struct Item {
         Buf<dbl4> *b;
         double *out;
         int k;
     } items[] = {{&c->x, x, 3}, {&c->v, v, 3}, {&c->q, quat, 4}, {&c->L, angmom, 3},
                  {&c->w, omega, 3}, {&c->f, f, 3}, {&c->t, torque, 3}};
+    SQCK(c->stage.alloc((size_t)22 * n));
+    double *plane = c->stage.p;
     for (auto &it : items) {
         if (!it.out) continue;
-        SQCK(cudaMemcpyAsync(h.data(), it.b->p, sizeof(dbl4) * n, cudaMemcpyDeviceToHost, c->st));
-        SQCK(cudaStreamSynchronize(c->st));
-        for (int i = 0; i < n; i++) {
-            const double r[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
-            for (int k = 0; k < it.k; k++) it.out[it.k * i + k] = r[k];
-        }
+        k_sq_unpack<<<nb(n), kB, 0, c->st>>>(it.b->p, n, it.k, plane);
+        SQCKL();
+        SQCK(cudaMemcpyAsync(it.out, plane, sizeof(double) * it.k * n, cudaMemcpyDeviceToHost, c->st));
+        plane += (size_t)it.k * n;
     }
+    SQCK(cudaStreamSynchronize(c->st));
     return 0;
 }
 
