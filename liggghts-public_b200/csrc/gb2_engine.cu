@@ -1044,15 +1044,17 @@ int do_build(gb2_ctx *c)
                                        endbit, c->st));
     bytes = c->cubtmp.n;
     CK(cub::DeviceScan::ExclusiveSum(c->cubtmp.p, bytes, c->counts.p, c->bin_start.p, c->mbins + 1, c->st));
-    // the list and its reverse, checked together (an overflowing list is cut
-    // at its capacity, so the reverse fill is safe and simply done again)
+    // the list and its reverse, checked together (either is cut at its
+    // capacity, so an overflowing build is safe and simply done again)
     for (int attempt = 0;; attempt++) {
         if (clear_status(c)) return GB2_ERR_CUDA;
         CK(cudaMemsetAsync(c->rnum.p, 0, sizeof(int) * c->cap, c->st));
         D = make_dev(c);
-        k_build_list<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
-        CKL();
-        k_rev_fill<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
+        // eight lanes per atom where the bins hold more than ~4 atoms on average
+        if ((long)nall >= 4l * c->mbins)
+            k_build_list<8><<<nblk(8l * c->nlocal), kBlock, 0, c->st>>>(D);
+        else
+            k_build_list<1><<<nblk(c->nlocal), kBlock, 0, c->st>>>(D);
         CKL();
         int st;
         if (read_status(c, &st)) return GB2_ERR_CUDA;

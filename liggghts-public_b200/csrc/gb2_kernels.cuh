@@ -321,11 +321,24 @@ __global__ void k_bin_keys(Dev D, int nall, unsigned *keys, int *vals, int *coun
 
 // Neighbor::granular_bin_no_newton (src/neigh_gran.cpp:485-639): half list
 // j > i in stencil order, ascending index within each bin, with the shear
-// history restored from the partner records of pairs touching now.
+// history restored from the partner records of pairs touching now; every
+// entry whose partner is owned joins that atom's reverse list at once
+// (unordered: k_rev_sort orders it).
+//
+// G lanes per atom test G consecutive candidates at a time; a ballot over the
+// atom's lanes keeps the list order.  One lane where a bin holds an atom or
+// two, so that a run of the stencil is a handful of candidates (20,000-sphere
+// pour: eight lanes are no faster).  Eight lanes where the bins are crowded:
+// small spheres binned at a large one's cutoff have ~9,000 candidates each,
+// one long serial walk (8,000 spheres, setup 5.4 -> 2.2 ms).
+template <int G>
 __global__ void k_build_list(Dev D)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = gi / G, g = gi % G;
     if (i >= D.nlocal) return;
+    const int lane0 = (threadIdx.x & 31) - g;                       // the atom's first lane
+    const unsigned gmask = (G == 32 ? ~0u : (1u << G) - 1u) << lane0;
     const int cap = D.cap;
     const dbl4 pi = D.pos[i];
     const double xtmp = pi.x, ytmp = pi.y, ztmp = pi.z, radi = pi.w;
@@ -340,41 +353,62 @@ __global__ void k_build_list(Dev D)
         const int b0 = max(ibin + run.x, 0), b1 = min(ibin + run.x + run.y, D.mbins);
         if (b0 >= b1) continue;
         const int e0 = D.bin_start[b0], e1 = D.bin_start[b1];
-        for (int q = e0; q < e1; q++) {
-            const int j = D.bin_atoms[q];
-            if (j <= i) continue;
-            const dbl4 pj = D.pos[j];
-            const double delx = xtmp - pj.x;
-            const double dely = ytmp - pj.y;
-            const double delz = ztmp - pj.z;
-            const double rsq = delx * delx + dely * dely + delz * delz;
-            const double radsum = (radi + pj.w) * 1.0;
-            const double cutsq = (radsum + skin) * (radsum + skin);
-            if (rsq <= cutsq) {
-                if (n < D.maxn) {
-                    const int e = n * cap + i;
-                    D.nbr[e] = j;
-                    int fl = 0;
-                    double h0 = 0.0, h1 = 0.0, h2 = 0.0;
-                    if (rsq < radsum * radsum) {
-                        const int tj = D.tag[j];
-                        for (int m = 0; m < np; m++)
-                            if (D.ptag[m * cap + i] == tj) {
-                                fl = 1;
-                                h0 = D.phist[(3 * m + 0) * cap + i];
-                                h1 = D.phist[(3 * m + 1) * cap + i];
-                                h2 = D.phist[(3 * m + 2) * cap + i];
-                                break;
-                            }
-                    }
-                    D.flag[e] = fl;
-                    // both history buffers, so either can serve as the next read buffer
-                    D.hist[e] = D.hist_out[e] = dbl4{h0, h1, h2, 0.0};
+        for (int base = e0; base < e1; base += G) {
+            const int q = base + g;
+            const int j = q < e1 ? D.bin_atoms[q] : -1;
+            bool take = false;
+            double rsq = 0.0, radsum = 0.0;
+            if (j > i) {
+                const dbl4 pj = D.pos[j];
+                const double delx = xtmp - pj.x;
+                const double dely = ytmp - pj.y;
+                const double delz = ztmp - pj.z;
+                rsq = delx * delx + dely * dely + delz * delz;
+                radsum = (radi + pj.w) * 1.0;
+                const double cutsq = (radsum + skin) * (radsum + skin);
+                take = rsq <= cutsq;
+            }
+            int slot = n;
+            if constexpr (G > 1) {
+                const unsigned m = __ballot_sync(gmask, take) >> lane0;
+                slot += __popc(m & ((1u << g) - 1u));
+                n += __popc(m);
+            } else {
+                n += take ? 1 : 0;
+            }
+            if (take && slot < D.maxn) {
+                const int e = slot * cap + i;
+                D.nbr[e] = j;
+                int fl = 0;
+                double h0 = 0.0, h1 = 0.0, h2 = 0.0;
+                if (rsq < radsum * radsum) {
+                    const int tj = D.tag[j];
+                    for (int m = 0; m < np; m++)
+                        if (D.ptag[m * cap + i] == tj) {
+                            fl = 1;
+                            h0 = D.phist[(3 * m + 0) * cap + i];
+                            h1 = D.phist[(3 * m + 1) * cap + i];
+                            h2 = D.phist[(3 * m + 2) * cap + i];
+                            break;
+                        }
                 }
-                n++;
+                D.flag[e] = fl;
+                // both history buffers, so either can serve as the next read buffer
+                D.hist[e] = D.hist_out[e] = dbl4{h0, h1, h2, 0.0};
+                if (j < D.nlocal) {
+                    const int r = atomicAdd(&D.rnum[j], 1);
+                    if (r < D.maxr) {
+                        D.rev[r * cap + j] = i;
+                        D.revs[r * cap + j] = (uint8_t)slot;
+                    } else {
+                        atomicOr(D.status, ST_REV_OVERFLOW);
+                        atomicMax(&D.need[2], r + 1);
+                    }
+                }
             }
         }
     }
+    if (g != 0) return;
     if (n > D.maxn) {
         atomicOr(D.status, ST_NEIGH_OVERFLOW);
         atomicMax(&D.need[0], n);
@@ -389,48 +423,76 @@ __global__ void k_build_list(Dev D)
     D.xhold[i] = h;
 }
 
-// reverse list: every local j collects the slots (i, s) with nbr == j
-__global__ void k_rev_fill(Dev D)
+// Order each reverse segment by owner index (the reference loop order; a
+// segment holds an owner once).  A thread sorts its atom's segment, up to 64
+// entries, by insertion in shared memory -- in global memory every exchange
+// was a dependent load and store -- and the block ranks each longer one
+// together.
+constexpr int kRevRow = 64;
+
+__global__ void __launch_bounds__(128) k_rev_sort(Dev D)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.nlocal) return;
-    const int cap = D.cap;
-    const int nn = D.nnum[i];
-    for (int s = 0; s < nn; s++) {
-        const int e = s * cap + i;
-        const int j = D.nbr[e];
-        if (j >= D.nlocal) continue;
-        const int r = atomicAdd(&D.rnum[j], 1);
-        if (r < D.maxr) {
-            D.rev[r * cap + j] = i;
-            D.revs[r * cap + j] = (uint8_t)s;
-        } else {
-            atomicOr(D.status, ST_REV_OVERFLOW);
-            atomicMax(&D.need[2], r + 1);
+    __shared__ int so[kRevRow * 128];
+    __shared__ uint8_t ss[kRevRow * 128];
+    __shared__ int longk[128], nlong;
+    const int tid = threadIdx.x, k = blockIdx.x * 128 + tid, cap = D.cap;
+    if (tid == 0) nlong = 0;
+    __syncthreads();
+    if (k < D.nlocal) {
+        const int n = min(D.rnum[k], D.maxr);
+        D.rnum[k] = n;
+        if (n > kRevRow) {
+            longk[atomicAdd(&nlong, 1)] = k;
+        } else if (n > 1) {
+            for (int a = 0; a < n; a++) {
+                const int ia = D.rev[a * cap + k];
+                const uint8_t sa = D.revs[a * cap + k];
+                int b = a - 1;
+                while (b >= 0 && so[b * 128 + tid] > ia) {
+                    so[(b + 1) * 128 + tid] = so[b * 128 + tid];
+                    ss[(b + 1) * 128 + tid] = ss[b * 128 + tid];
+                    b--;
+                }
+                so[(b + 1) * 128 + tid] = ia;
+                ss[(b + 1) * 128 + tid] = sa;
+            }
+            for (int a = 0; a < n; a++) {
+                D.rev[a * cap + k] = so[a * 128 + tid];
+                D.revs[a * cap + k] = ss[a * 128 + tid];
+            }
         }
     }
-}
-
-// order each reverse segment by owner index (the reference loop order)
-__global__ void k_rev_sort(Dev D)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= D.nlocal) return;
-    const int cap = D.cap;
-    int n = D.rnum[k];
-    if (n > D.maxr) n = D.maxr;
-    D.rnum[k] = n;
-    for (int a = 1; a < n; a++) {
-        const int ia = D.rev[a * cap + k];
-        const uint8_t sa = D.revs[a * cap + k];
-        int b = a - 1;
-        while (b >= 0 && D.rev[b * cap + k] > ia) {
-            D.rev[(b + 1) * cap + k] = D.rev[b * cap + k];
-            D.revs[(b + 1) * cap + k] = D.revs[b * cap + k];
-            b--;
+    __syncthreads();
+    for (int q = 0; q < nlong; q++) {   // segments of one block are independent of each other's order
+        const int kk = longk[q], n = D.rnum[kk];
+        if (n <= kRevRow * 128) {
+            for (int e = tid; e < n; e += 128) {
+                so[e] = D.rev[e * cap + kk];
+                ss[e] = D.revs[e * cap + kk];
+            }
+            __syncthreads();
+            for (int e = tid; e < n; e += 128) {
+                const int v = so[e];
+                int rank = 0;
+                for (int f = 0; f < n; f++) rank += so[f] < v ? 1 : 0;
+                D.rev[rank * cap + kk] = v;
+                D.revs[rank * cap + kk] = ss[e];
+            }
+        } else if (tid == 0) {   // longer than the shared rows: insertion in place
+            for (int a = 1; a < n; a++) {
+                const int ia = D.rev[a * cap + kk];
+                const uint8_t sa = D.revs[a * cap + kk];
+                int b = a - 1;
+                while (b >= 0 && D.rev[b * cap + kk] > ia) {
+                    D.rev[(b + 1) * cap + kk] = D.rev[b * cap + kk];
+                    D.revs[(b + 1) * cap + kk] = D.revs[b * cap + kk];
+                    b--;
+                }
+                D.rev[(b + 1) * cap + kk] = ia;
+                D.revs[(b + 1) * cap + kk] = sa;
+            }
         }
-        D.rev[(b + 1) * cap + k] = ia;
-        D.revs[(b + 1) * cap + k] = sa;
+        __syncthreads();
     }
 }
 
