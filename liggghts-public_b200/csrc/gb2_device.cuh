@@ -503,6 +503,11 @@ __device__ __forceinline__ void wall_record_put(WallRec *rec, int &n, const Cont
     n++;
 }
 
+// The wall histories (whist, shist, spartner, snp) are read from L2: the tail
+// kernel reads them before it has waited for the grid it depends on, and two
+// atoms whose words share a line may be handled on different SMs from one step
+// to the next.
+//
 // One candidate triangle t in contact with atom i (deltan <= 0): the body of
 // FixWallGran::post_force_mesh's loop -- FixContactHistoryMesh::handleContact
 // (slot lookup, new slot with the shear of a coplanar neighbour for face
@@ -555,9 +560,9 @@ static __device__ bool mesh_contact(const Dev &D, const MeshDev &M, int i, int t
             for (int k = 0; k < nn; k++) {
                 const int tri = sp[k];
                 if (tri >= 0 && tri != t && coplanar_node_neighs(M, tri, t)) {
-                    h0 = M.shist[(3 * k + 0) * cap + i];
-                    h1 = M.shist[(3 * k + 1) * cap + i];
-                    h2 = M.shist[(3 * k + 2) * cap + i];
+                    h0 = __ldcg(&M.shist[(3 * k + 0) * cap + i]);
+                    h1 = __ldcg(&M.shist[(3 * k + 1) * cap + i]);
+                    h2 = __ldcg(&M.shist[(3 * k + 2) * cap + i]);
                 }
             }
         }
@@ -566,8 +571,8 @@ static __device__ bool mesh_contact(const Dev &D, const MeshDev &M, int i, int t
         M.shist[(3 * ic + 2) * cap + i] = h2;
         slot = ic;
     }
-    double sh[3] = {M.shist[(3 * slot + 0) * cap + i], M.shist[(3 * slot + 1) * cap + i],
-                    M.shist[(3 * slot + 2) * cap + i]};
+    double sh[3] = {__ldcg(&M.shist[(3 * slot + 0) * cap + i]), __ldcg(&M.shist[(3 * slot + 1) * cap + i]),
+                    __ldcg(&M.shist[(3 * slot + 2) * cap + i])};
     const double dvec[3] = {-delta[0], -delta[1], -delta[2]};
     double vwall[3] = {0.0, 0.0, 0.0};
     if (M.vnode) {   // moving mesh: barycentric node velocity (src/fix_wall_gran.cpp:992-996)
@@ -644,7 +649,7 @@ __device__ __forceinline__ void mesh_wall_items(const Dev &D, const MeshDev &M, 
     const int lane = threadIdx.x & 31;
     const int cap = D.cap;
     const int nn = own ? M.tcnt[i] : 0;
-    int np = own ? M.snp[i] : 0;
+    int np = own ? __ldcg(&M.snp[i]) : 0;
     const WarpItems it = warp_items_cnt(nn);
     if (it.total == 0) return;
     unsigned long long touch = 0ull;
@@ -661,7 +666,7 @@ __device__ __forceinline__ void mesh_wall_items(const Dev &D, const MeshDev &M, 
             double delta[3], bary[3] = {0., 0., 0.};
             int barysign = -1;
             const int t = M.tlist[(wq - exL) * cap + iL];
-            sp[wq] = M.spartner[(wq - exL) * cap + iL];
+            sp[wq] = __ldcg(&M.spartner[(wq - exL) * cap + iL]);
             const double deltan = tri_sphere(M.tri[t], pr, cs, delta, barysign, 1e-8, bary);
             hit = !(deltan > D.cutneighmax) && (deltan <= 0);
         }
@@ -789,7 +794,7 @@ __device__ __forceinline__ bool plane_wall_atom(const Dev &D, const FixDev &F, i
     }
     if (deltan > D.cutneighmax) return false;
     if (deltan <= 0) {
-        double sh[3] = {F.whist[0 * cap + i], F.whist[1 * cap + i], F.whist[2 * cap + i]};
+        double sh[3] = {__ldcg(&F.whist[0 * cap + i]), __ldcg(&F.whist[1 * cap + i]), __ldcg(&F.whist[2 * cap + i])};
         const double vwall[3] = {0., 0., 0.};
         wall_contact(mat(D, ti, F.wtype), d, -deltan, pi.w, vi, wi, vwall, mass, sh, upd, D.dt, F.rolling != 0,
                      D.tdamp != 0, acc);

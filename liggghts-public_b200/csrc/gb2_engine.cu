@@ -161,7 +161,7 @@ struct gb2_ctx {
     DBuf<dbl4> pos, vel, omg, pos2, vel2, omg2, f, tq, tailf, tailt, xhold;
     bool split = false;           // GB2_PREC_SPLIT
     DBuf<flt8> kin, kin2;         // split precision: FP32 kinematics records (double-buffered like vel)
-    DBuf<uint8_t> revs;
+    DBuf<uint8_t> revs, tflag;
     int nsm = 148;                // SMs of the device
     int tail_per_sm = 8;          // blocks of the tail kernel per SM (kTailAtoms atoms per warp)
     int item_cap = 160;           // listed-round capacity per warp and side (grown on demand up to kItemCap)
@@ -387,6 +387,7 @@ Dev make_dev(gb2_ctx *c)
     D.tq = c->tq.p;
     D.tailf = c->tailf.p;
     D.tailt = c->tailt.p;
+    D.tflag = c->tflag.p;
     D.tail = c->tail.p;
     D.tailcnt = c->dtailcnt.p;
     D.xhold = c->xhold.p;
@@ -1569,6 +1570,7 @@ int gb2_upload_atoms(gb2_ctx *c, int n, const double *x, const double *v, const 
     CK(c->tailf.alloc(cap));
     CK(c->tailt.alloc(cap));
     CK(c->tail.alloc(cap));
+    CK(c->tflag.alloc(cap));
     CK(c->xhold.alloc(cap));
     CK(c->nnum.alloc(cap));
     CK(c->rnum.alloc(cap));
@@ -1787,6 +1789,7 @@ static int reserve_cap(gb2_ctx *c, int want)
     CK(c->tailf.alloc(cap));
     CK(c->tailt.alloc(cap));
     CK(c->tail.alloc(cap));
+    CK(c->tflag.alloc(cap));
     CK(c->xhold.alloc(cap));
     CK(c->nnum.alloc(cap));
     CK(c->rnum.alloc(cap));

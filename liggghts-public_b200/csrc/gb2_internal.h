@@ -7,7 +7,7 @@
 //     omg  {wx, wy, wz, -}        type, tag (int32)
 //   per owned atom:
 //     f, tq {., ., ., -}          force / torque of the last step
-//     tail[w]                     atoms finished by the tail kernel (wall candidates or
+//     tail[w], tflag[i]           atoms finished by the tail kernel (wall candidates or
 //                                 more than 64 entries on a side), listed at each build
 //     tailf, tailt                their pair sums, left by the pair step kernel
 //     xhold {x, y, z, -}          positions at the last neighbour build
@@ -129,6 +129,7 @@ struct Dev {
     int *type, *tag;
     dbl4 *f, *tq, *tailf, *tailt, *xhold;
     int *tail, *tailcnt;   // tail-kernel atom list and its length
+    uint8_t *tflag;        // per owned atom: on that list
     // half list
     int maxn;
     int item_cap;          // per-warp list capacity of the pair step's listed rounds (<= kItemCap)

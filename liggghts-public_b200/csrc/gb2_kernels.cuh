@@ -972,7 +972,9 @@ __global__ void k_tail_list(Dev D)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= D.nlocal) return;
-    if (tail_atom(D, k, D.rnum[k], D.nnum[k])) D.tail[atomicAdd(D.tailcnt, 1)] = k;
+    const bool tail = tail_atom(D, k, D.rnum[k], D.nnum[k]);
+    D.tflag[k] = tail ? 1 : 0;
+    if (tail) D.tail[atomicAdd(D.tailcnt, 1)] = k;
 }
 
 // Start of a queue of steps: the step just run (not queued) may already

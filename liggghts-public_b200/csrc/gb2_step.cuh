@@ -11,7 +11,10 @@ namespace gb2 {
 // Programmatic dependent launch: the pair step lets the tail kernel be
 // scheduled as soon as all of its blocks are running; the tail kernel does
 // what does not need the pair sums first and then waits for the pair step
-// to complete (all its memory operations visible).
+// to complete (all its memory operations visible).  The next step's pair step
+// is the tail kernel's dependent in turn: it may start early, but lets its own
+// tail kernel start only after it has waited, so a tail kernel never runs
+// beside the previous step's.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -392,8 +395,6 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     // each round's owner-lane masks, tagged with the round
     extern __shared__ __align__(16) unsigned char pair_dyn[];
     __shared__ unsigned long long sgrp[4][32];
-    grid_dep_launch();   // the tail kernel may be scheduled once every block of this grid runs
-    if (step_cancelled(D)) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) / G;   // G lanes per atom, the first owns it
     const int wbase = (blockIdx.x * blockDim.x + wid * 32) / G;
@@ -405,6 +406,17 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     int nr = 0, nn = 0;
     unsigned long long mrev = 0ull, mown = 0ull;
     bool serial = false, tail = false;
+    // what changes only at a build is read while the previous step's tail
+    // kernel still runs (this grid is its programmatic dependent)
+    if (valid) {
+        nr = D.rnum[k];
+        nn = D.nnum[k];
+        tail = D.tflag[k] != 0;
+        serial = nr > 64 || nn > 64;
+    }
+    grid_dep_wait();
+    grid_dep_launch();   // the tail kernel may be scheduled once every block of this grid runs
+    if (step_cancelled(D)) return;
     if (valid) {
         // the atom's own records, including those only the tail needs, are
         // requested first so their latency overlaps the screening
@@ -414,10 +426,6 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
             if (fuse_next) stage4(&stail[2][threadIdx.x], &D.xhold[k]);
         }
         pk = D.pos[k];
-        nr = D.rnum[k];
-        nn = D.nnum[k];
-        serial = nr > 64 || nn > 64;
-        tail = tail_atom(D, k, nr, nn);
         if (!serial && upd) prevm = D.prevmask[k];
     }
     // screening of every non-serial atom of the warp, listing its touching
@@ -604,6 +612,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ De
             }
         }
         grid_dep_wait();
+        grid_dep_launch();   // the next step's pair step may be scheduled (it waits for this grid)
         ContactOut acc;
         for (int c = 0; c < 3; c++) acc.F[c] = acc.T[c] = 0.0;
         if (own) {
@@ -655,46 +664,51 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ De
 // Host side: the pair step with one or two lanes per atom.  Registers: 5
 // blocks per SM (96) for one lane, where the chip is full; 4 (128, no spill)
 // for two, where it is not.
-template <bool ROLLING, bool SPLIT, bool ONE>
-inline void launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                            int store_f, size_t smem)
-{
-    const auto kernel = lanes == 1 ? k_pair_step<ROLLING, 5, SPLIT, ONE, 1> : k_pair_step<ROLLING, 4, SPLIT, ONE, 2>;
-    const int nblocks = (int)(((long)D.nlocal * lanes + 127) / 128);
-    kernel<<<nblocks, 128, smem, st>>>(D, shearupdate, integrate, fuse_next, store_f);
-}
-
-template <bool SPLIT>
-inline void launch_pair_step(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                             int store_f, size_t smem)
-{
-    if (D.rolling && D.ntypes == 1)
-        launch_pair_one<true, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
-    else if (D.rolling)
-        launch_pair_one<true, SPLIT, false>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
-    else if (D.ntypes == 1)
-        launch_pair_one<false, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
-    else
-        launch_pair_one<false, SPLIT, false>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
-}
-
-// Host side: the tail kernel launched as a programmatic dependent of the
-// pair step launched just before it on the same stream.
-template <bool ROLLING, bool SPLIT>
-inline cudaError_t launch_pair_tail(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate,
-                                    int fuse_next, int store_f)
+template <typename Kernel>
+inline cudaError_t launch_dependent(Kernel kernel, int nblocks, size_t smem, cudaStream_t st, const Dev &D,
+                                    int shearupdate, int integrate, int fuse_next, int store_f)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nblocks);
     cfg.blockDim = dim3(128);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_pair_tail<ROLLING, SPLIT>, D, shearupdate, integrate, fuse_next, store_f);
+    return cudaLaunchKernelEx(&cfg, kernel, D, shearupdate, integrate, fuse_next, store_f);
+}
+
+template <bool ROLLING, bool SPLIT, bool ONE>
+inline cudaError_t launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
+                            int store_f, size_t smem)
+{
+    const auto kernel = lanes == 1 ? k_pair_step<ROLLING, 5, SPLIT, ONE, 1> : k_pair_step<ROLLING, 4, SPLIT, ONE, 2>;
+    const int nblocks = (int)(((long)D.nlocal * lanes + 127) / 128);
+    return launch_dependent(kernel, nblocks, smem, st, D, shearupdate, integrate, fuse_next, store_f);
+}
+
+template <bool SPLIT>
+inline cudaError_t launch_pair_step(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
+                             int store_f, size_t smem)
+{
+    if (D.rolling && D.ntypes == 1)
+        return launch_pair_one<true, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    if (D.rolling)
+        return launch_pair_one<true, SPLIT, false>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    if (D.ntypes == 1)
+        return launch_pair_one<false, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    return launch_pair_one<false, SPLIT, false>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+}
+
+// Host side: the tail kernel of the pair step launched just before it.
+template <bool ROLLING, bool SPLIT>
+inline cudaError_t launch_pair_tail(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate,
+                                    int fuse_next, int store_f)
+{
+    return launch_dependent(k_pair_tail<ROLLING, SPLIT>, nblocks, 0, st, D, shearupdate, integrate, fuse_next, store_f);
 }
 
 }  // namespace gb2
