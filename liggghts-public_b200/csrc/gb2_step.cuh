@@ -18,6 +18,8 @@ namespace gb2 {
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // A kernel of a step queued ahead returns at once when an earlier step has
 // asked for a neighbour rebuild (that step's successors are redone after it).
 __device__ __forceinline__ bool step_cancelled(const Dev &D) { return D.dstop && *(volatile int *)D.dstop < D.step; }
@@ -453,6 +455,22 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
         for (int base = 0; base < tot; base += 32, round++) {
             const int w = base + lane;
             int L = -1 - lane;   // lanes without an item match nobody
+            // the next round's records on their way to L1 while this round's
+            // arithmetic runs (bed of 2M spheres 847 -> 815 us/step, 1M hopper
+            // unchanged; the same from the screening loop, or to L2 only, evicts
+            // what the current round needs)
+            if (w + 32 < tot) {
+                const bool own = w + 32 >= nlrev;
+                const int2 item = own ? lown[w + 32 - nlrev] : lrev[w + 32];
+                const int hrow = own ? wbase + (item.y & 31) / G : item.x;
+                if constexpr (SPLIT) {
+                    prefetch_l1(&D.kin[item.x]);
+                } else {
+                    prefetch_l1(&D.vel[item.x]);
+                    prefetch_l1(&D.omg[item.x]);
+                }
+                prefetch_l1(&D.hist[(item.y >> 8) * cap + hrow]);
+            }
             if (w < tot) {
                 const bool own = w >= nlrev;
                 const int2 item = own ? lown[w - nlrev] : lrev[w];
@@ -661,9 +679,8 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ De
     grid_dep_wait();
 }
 
-// Host side: the pair step with one or two lanes per atom.  Registers: 5
-// blocks per SM (96) for one lane, where the chip is full; 4 (128, no spill)
-// for two, where it is not.
+// Host side: a kernel launched as a programmatic dependent of the one before it
+// on the same stream.
 template <typename Kernel>
 inline cudaError_t launch_dependent(Kernel kernel, int nblocks, size_t smem, cudaStream_t st, const Dev &D,
                                     int shearupdate, int integrate, int fuse_next, int store_f)
@@ -681,11 +698,16 @@ inline cudaError_t launch_dependent(Kernel kernel, int nblocks, size_t smem, cud
     return cudaLaunchKernelEx(&cfg, kernel, D, shearupdate, integrate, fuse_next, store_f);
 }
 
+// The pair step with one or two lanes per atom.  Registers: FP64 takes 4 blocks
+// per SM (128 registers, no spill): 5 blocks (96) spill 20 doubles through the
+// L1 that the gathers need, 3 leave too few warps (hopper of 1M 253, 267 and
+// 307 us/step, bed of 2M 847, 907 and 847).  Split precision fits 6 blocks (80):
+// 206 us/step against 209 with 5 and 240 with 4.
 template <bool ROLLING, bool SPLIT, bool ONE>
 inline cudaError_t launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
                             int store_f, size_t smem)
 {
-    const auto kernel = lanes == 1 ? k_pair_step<ROLLING, 5, SPLIT, ONE, 1> : k_pair_step<ROLLING, 4, SPLIT, ONE, 2>;
+    const auto kernel = lanes == 1 ? k_pair_step<ROLLING, SPLIT ? 6 : 4, SPLIT, ONE, 1> : k_pair_step<ROLLING, 4, SPLIT, ONE, 2>;
     const int nblocks = (int)(((long)D.nlocal * lanes + 127) / 128);
     return launch_dependent(kernel, nblocks, smem, st, D, shearupdate, integrate, fuse_next, store_f);
 }
