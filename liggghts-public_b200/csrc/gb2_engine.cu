@@ -191,8 +191,8 @@ struct gb2_ctx {
     std::vector<int> h_stencil;
     std::vector<int2> h_srow;   // stencil runs {first offset, bins}
     DBuf<int2> srow;
-    DBuf<int> stencil, bin_start, bin_atoms, counts, vals, vals2, sel, nsel;
-    DBuf<unsigned> keys, keys2;
+    DBuf<int> stencil, bin_start, bin_atoms, counts, vals, vals2, arrivals, sort_counts, sort_start, sel, nsel;
+    DBuf<unsigned> keys;
     DBuf<uint8_t> bflags;
     DBuf<char> cubtmp;
     DBuf<int> dstatus, ddflag, dneed, dtailcnt;
@@ -901,6 +901,25 @@ int do_partners(gb2_ctx *c)
     return set_err(c, GB2_ERR_CAPACITY, "contact history partner capacity could not be grown");
 }
 
+// out: the n atoms of keys (bin) and vals (arrival in its bin) in bin order,
+// ascending within a bin; start[nbins + 1] the scan of counts
+int bin_order(gb2_ctx *c, int n, size_t nbins, const int *counts, int *start, int *out)
+{
+    size_t bytes = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, bytes, counts, start, (int)nbins + 1, c->st);
+    if (cub_tmp(c, bytes)) return GB2_ERR_CUDA;
+    bytes = c->cubtmp.n;
+    CK(cub::DeviceScan::ExclusiveSum(c->cubtmp.p, bytes, counts, start, (int)nbins + 1, c->st));
+    CK(c->arrivals.alloc(std::max(c->nmax, 1)));
+    if (n > 0) {
+        k_bin_scatter<<<nblk(n), kBlock, 0, c->st>>>(n, c->keys.p, c->vals.p, start, c->arrivals.p);
+        CKL();
+        k_bin_rank<<<nblk(n), kBlock, 0, c->st>>>(n, c->keys.p, start, counts, c->arrivals.p, out);
+        CKL();
+    }
+    return 0;
+}
+
 int do_atom_sort(gb2_ctx *c)
 {
     // Atom::sort (src/atom.cpp:1309): stable order by spatial sort bin
@@ -909,18 +928,17 @@ int do_atom_sort(gb2_ctx *c)
     const int n = c->nlocal;
     Dev D = make_dev(c);
     CK(c->keys.alloc(std::max(c->nmax, 1)));
-    CK(c->keys2.alloc(std::max(c->nmax, 1)));
     CK(c->vals.alloc(std::max(c->nmax, 1)));
     CK(c->vals2.alloc(std::max(c->nmax, 1)));
+    const size_t nbins = (size_t)c->snb[0] * c->snb[1] * c->snb[2];
+    CK(c->sort_counts.alloc(nbins + 1));
+    CK(c->sort_start.alloc(nbins + 1));
+    CK(cudaMemsetAsync(c->sort_counts.p, 0, sizeof(int) * (nbins + 1), c->st));
     k_sort_keys<<<nblk(n), kBlock, 0, c->st>>>(D, c->slo[0], c->slo[1], c->slo[2], c->sinv[0], c->sinv[1], c->sinv[2],
-                                                c->snb[0], c->snb[1], c->snb[2], c->keys.p, c->vals.p);
+                                                c->snb[0], c->snb[1], c->snb[2], c->keys.p, c->vals.p,
+                                                c->sort_counts.p);
     CKL();
-    size_t bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, bytes, c->keys.p, c->keys2.p, c->vals.p, c->vals2.p, n, 0, 32, c->st);
-    if (cub_tmp(c, bytes)) return GB2_ERR_CUDA;
-    bytes = c->cubtmp.n;
-    CK(cub::DeviceRadixSort::SortPairs(c->cubtmp.p, bytes, c->keys.p, c->keys2.p, c->vals.p, c->vals2.p, n, 0, 32,
-                                       c->st));
+    if (bin_order(c, n, nbins, c->sort_counts.p, c->sort_start.p, c->vals2.p)) return GB2_ERR_CUDA;
     const int *perm = c->vals2.p;
     // every per-atom array moves with its atom: gather into a persistent
     // shadow buffer and swap (no allocation once the shadows exist)
@@ -1025,7 +1043,6 @@ int do_build(gb2_ctx *c)
 {
     const int nall = c->nlocal + c->nghost;
     CK(c->keys.alloc(std::max(c->nmax, 1)));
-    CK(c->keys2.alloc(std::max(c->nmax, 1)));
     CK(c->vals.alloc(std::max(c->nmax, 1)));
     CK(c->bin_atoms.alloc(std::max(c->nmax, 1)));
     CK(cudaMemsetAsync(c->counts.p, 0, sizeof(int) * ((size_t)c->mbins + 1), c->st));
@@ -1033,18 +1050,7 @@ int do_build(gb2_ctx *c)
     Dev D = make_dev(c);
     k_bin_keys<<<nblk(nall), kBlock, 0, c->st>>>(D, nall, c->keys.p, c->vals.p, c->counts.p);
     CKL();
-    size_t bytes = 0, b2 = 0;
-    int endbit = 1;
-    while ((1l << endbit) < (long)c->mbins + 1) endbit++;
-    cub::DeviceRadixSort::SortPairs(nullptr, bytes, c->keys.p, c->keys2.p, c->vals.p, c->bin_atoms.p, nall, 0, endbit,
-                                    c->st);
-    cub::DeviceScan::ExclusiveSum(nullptr, b2, c->counts.p, c->bin_start.p, c->mbins + 1, c->st);
-    if (cub_tmp(c, std::max(bytes, b2))) return GB2_ERR_CUDA;
-    bytes = c->cubtmp.n;
-    CK(cub::DeviceRadixSort::SortPairs(c->cubtmp.p, bytes, c->keys.p, c->keys2.p, c->vals.p, c->bin_atoms.p, nall, 0,
-                                       endbit, c->st));
-    bytes = c->cubtmp.n;
-    CK(cub::DeviceScan::ExclusiveSum(c->cubtmp.p, bytes, c->counts.p, c->bin_start.p, c->mbins + 1, c->st));
+    if (bin_order(c, nall, c->mbins, c->counts.p, c->bin_start.p, c->bin_atoms.p)) return GB2_ERR_CUDA;
     // the list and its reverse, checked together (either is cut at its
     // capacity, so an overflowing build is safe and simply done again)
     for (int attempt = 0;; attempt++) {

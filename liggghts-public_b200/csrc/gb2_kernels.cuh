@@ -209,7 +209,7 @@ __global__ void k_pbc(Dev D, double lo0, double lo1, double lo2, double hi0, dou
 
 // Atom::sort keys (src/atom.cpp:1343-1354)
 __global__ void k_sort_keys(Dev D, double lo0, double lo1, double lo2, double inv0, double inv1, double inv2, int nb0,
-                            int nb1, int nb2, unsigned *keys, int *vals)
+                            int nb1, int nb2, unsigned *keys, int *vals, int *counts)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= D.nlocal) return;
@@ -223,8 +223,33 @@ __global__ void k_sort_keys(Dev D, double lo0, double lo1, double lo2, double in
     ix = min(ix, nb0 - 1);
     iy = min(iy, nb1 - 1);
     iz = min(iz, nb2 - 1);
-    keys[i] = static_cast<unsigned>(iz * nb1 * nb0 + iy * nb0 + ix);
-    vals[i] = i;
+    const int b = iz * nb1 * nb0 + iy * nb0 + ix;
+    keys[i] = static_cast<unsigned>(b);
+    vals[i] = atomicAdd(&counts[b], 1);   // its place among the bin's arrivals
+}
+
+// The atoms in bin order, ascending within a bin: a counting sort whose
+// arrival order (k_bin_scatter; start is the scan of the counts) is replaced
+// by the rank of each atom among its bin's (k_bin_rank).  Bins hold an atom or
+// two, so this reads and writes each atom a few times where a radix sort takes
+// three or four passes of ~10 us even for a thousand atoms.
+__global__ void k_bin_scatter(int n, const unsigned *__restrict__ keys, const int *__restrict__ arrival,
+                              const int *__restrict__ start, int *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[start[keys[i]] + arrival[i]] = i;
+}
+
+__global__ void k_bin_rank(int n, const unsigned *__restrict__ keys, const int *__restrict__ start,
+                           const int *__restrict__ counts, const int *__restrict__ in, int *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const unsigned b = keys[i];
+    const int s = start[b], m = counts[b];
+    int rank = 0;
+    for (int q = 0; q < m; q++) rank += in[s + q] < i ? 1 : 0;
+    out[s + rank] = i;
 }
 
 template <typename T>
@@ -315,8 +340,7 @@ __global__ void k_bin_keys(Dev D, int nall, unsigned *keys, int *vals, int *coun
         b = b < 0 ? 0 : D.mbins - 1;
     }
     keys[i] = static_cast<unsigned>(b);
-    vals[i] = i;
-    atomicAdd(&counts[b], 1);
+    vals[i] = atomicAdd(&counts[b], 1);   // its place among the bin's arrivals
 }
 
 // Neighbor::granular_bin_no_newton (src/neigh_gran.cpp:485-639): half list
