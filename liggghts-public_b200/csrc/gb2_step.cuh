@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     // entries (all lanes take part in the list ballots)
     int nlrev = 0, nlown = 0;
     int2 *lrev = reinterpret_cast<int2 *>(pair_dyn) + (size_t)wid * 2 * D.item_cap, *lown = lrev + D.item_cap;
-    const bool listed = screen_list<G>(D, k, (valid && !serial) ? nr : 0, (valid && !serial) ? nn : 0, pk, mrev, mown,
+    const bool listed = screen_list<G, SPLIT ? 2 : 4>(D, k, (valid && !serial) ? nr : 0, (valid && !serial) ? nn : 0, pk, mrev, mown,
                                        lrev, lown, nlrev, nlown);
     if (!listed && lane == 0 && D.item_cap > 0) atomicAdd(&D.need[4], 1);   // lists too short: counted for the host
     // FP64 path: plain in-order sums (bit-exact).  Split path: FP32 sums of
