@@ -59,40 +59,32 @@ __device__ __forceinline__ double pow_pos(double base, double e)
     return r;
 }
 
-// 4x4 solve by Gaussian elimination with partial pivoting, rows exchanged by
-// selects so the matrix stays in registers; false if singular
-__device__ __forceinline__ bool solve4r(double a[4][5], double *x)
+// The Newton step: H x + c x4 = f, d.x = f4, with H symmetric (h: xx, xy, xz,
+// yy, yz, zz), by the cofactors of the bordered matrix,
+//   x = (f4 adj(H) c - d x (H (c x f))) / D,  x4 = (adj(H) d . f - det(H) f4) / D,
+//   D = d . adj(H) c  (minus the determinant of the 4x4 matrix),
+// which also holds for a singular H.  One division ends a chain of a dozen
+// multiply-adds; elimination with partial pivoting was four of each in
+// sequence, half of a trip's latency.  False when D is zero or not a number.
+__device__ __forceinline__ bool solve_bordered(const double *h, const double *c, const double *d, const double *f,
+                                               double f4, double *x)
 {
-    bool ok = true;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-#pragma unroll
-        for (int r = c + 1; r < 4; r++) {
-            const bool sw = fabs(a[r][c]) > fabs(a[c][c]);
-#pragma unroll
-            for (int j = c; j < 5; j++) {
-                const double t = a[c][j], u = a[r][j];
-                a[c][j] = sw ? u : t;
-                a[r][j] = sw ? t : u;
-            }
-        }
-        ok = ok && a[c][c] != 0.0;
-        const double inv = 1.0 / a[c][c];
-#pragma unroll
-        for (int j = c + 1; j < 5; j++) a[c][j] *= inv;
-#pragma unroll
-        for (int r = c + 1; r < 4; r++)
-#pragma unroll
-            for (int j = c + 1; j < 5; j++) a[r][j] -= a[r][c] * a[c][j];
-    }
-#pragma unroll
-    for (int i = 3; i >= 0; i--) {
-        double s = a[i][4];
-#pragma unroll
-        for (int j = i + 1; j < 4; j++) s -= a[i][j] * x[j];
-        x[i] = s;
-    }
-    return ok;
+    const double axx = h[3] * h[5] - h[4] * h[4], axy = h[2] * h[4] - h[1] * h[5], axz = h[1] * h[4] - h[2] * h[3];
+    const double ayy = h[0] * h[5] - h[2] * h[2], ayz = h[1] * h[2] - h[0] * h[4], azz = h[0] * h[3] - h[1] * h[1];
+    const double z[3] = {axx * c[0] + axy * c[1] + axz * c[2], axy * c[0] + ayy * c[1] + ayz * c[2],
+                         axz * c[0] + ayz * c[1] + azz * c[2]};
+    const double w[3] = {axx * d[0] + axy * d[1] + axz * d[2], axy * d[0] + ayy * d[1] + ayz * d[2],
+                         axz * d[0] + ayz * d[1] + azz * d[2]};
+    const double det = h[0] * axx + h[1] * axy + h[2] * axz;
+    double cf[3], r[3];
+    cross3(c, f, cf);
+    const double hv[3] = {h[0] * cf[0] + h[1] * cf[1] + h[2] * cf[2], h[1] * cf[0] + h[3] * cf[1] + h[4] * cf[2],
+                          h[2] * cf[0] + h[4] * cf[1] + h[5] * cf[2]};
+    cross3(d, hv, r);
+    const double D = dot3(d, z), inv = 1.0 / D;
+    for (int k = 0; k < 3; k++) x[k] = (f4 * z[k] - r[k]) * inv;
+    x[3] = (dot3(w, f) - det * f4) * inv;
+    return D != 0.0 && !isnan(D);
 }
 
 // the sum of v over the lanes of one body (4) or of the pair (8)
@@ -365,7 +357,7 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
                 merit1 = merit;
             }
             if (accept) {
-                if (fabs(before - res1) / fmax(before, res1) < 1e-3) converged = true;
+                if (fabs(before - res1) < 1e-3 * fmax(before, res1)) converged = true;
                 if (it >= maxit) fail = true;
                 if (converged || fail) end = true;
                 else step = true;
@@ -386,23 +378,20 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
         // ---- Newton steps (all lanes take part in the sums; the groups that asked use the result)
         if (__any_sync(FULL, step)) {
             const double w = second ? mu * mu * dcur : dcur;
-            double a[4][5];
             const double r0 = X.rc[0] * w, r1 = X.rc[1] * w;
-            a[0][0] = sum8(FULL, r0 * X.rc[0]);
-            a[0][1] = a[1][0] = sum8(FULL, r0 * X.rc[1]);
-            a[0][2] = a[2][0] = sum8(FULL, r0 * X.rc[2]);
-            a[1][1] = sum8(FULL, r1 * X.rc[1]);
-            a[1][2] = a[2][1] = sum8(FULL, r1 * X.rc[2]);
-            a[2][2] = sum8(FULL, X.rc[2] * w * X.rc[2]);
+            double h[6], cc[3], dd[3];
+            h[0] = sum8(FULL, r0 * X.rc[0]);
+            h[1] = sum8(FULL, r0 * X.rc[1]);
+            h[2] = sum8(FULL, r0 * X.rc[2]);
+            h[3] = sum8(FULL, r1 * X.rc[1]);
+            h[4] = sum8(FULL, r1 * X.rc[2]);
+            h[5] = sum8(FULL, X.rc[2] * w * X.rc[2]);
             for (int k = 0; k < 3; k++) {
-                a[k][3] = 2.0 * mu * gB[k];
-                a[3][k] = gA[k] - gB[k];
-                a[k][4] = F[k];
+                cc[k] = 2.0 * mu * gB[k];
+                dd[k] = gA[k] - gB[k];
             }
-            a[3][3] = 0.0;
-            a[3][4] = F[3];
             double x[4];
-            bool ok = solve4r(a, x);
+            bool ok = solve_bordered(h, cc, dd, F, F[3], x);
             for (int k = 0; k < 4; k++) ok = ok && !isnan(x[k]);
             if (step) {
                 it++;
