@@ -7,9 +7,9 @@
 // any particle moved more than skin/2, pair pass (screening of every
 // half-list slot, then the contact-point solves in work lists by kind),
 // deterministic per-particle sums (reverse slots in ascending owner order,
-// then own slots), final_integrate.
+// then own slots), final_integrate; the sums, final_integrate and the next
+// step's initial_integrate are one kernel.
 #include <cub/cub.cuh>
-#include <thrust/iterator/counting_iterator.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -311,8 +311,11 @@ struct gb2_sq_ctx {
     Buf<double> xs, red;
     Buf<char> tmp;
     Buf<unsigned long long> counters;
-    Buf<int> dflag;
-    int *h_pin = nullptr;
+    Buf<int> dflag, dstop;
+    int *h_pin = nullptr;     // [0] list length, [1] flag, [4] set by the device with dstop, [5] dstop read back
+    bool queued = false;      // a step's kernels look at dstop
+    int step = 0;
+    cudaEvent_t qev[3] = {};
     double Yeff = 0, Geff = 0, betaeff = 0, mu = 0;
     long nbuilds = 0;
     Buf<float> mlp;
@@ -321,7 +324,6 @@ struct gb2_sq_ctx {
     // work lists of the pair pass: 2 lists of nslots items, then the item
     // counts and the taken counter
     Buf<int> work;
-    Buf<signed char> kind;   // per slot: the work list the screen puts it on
     Buf<float4> guess;       // learned guesses of the first contacts, by list position
     Buf<double> stage;       // particle upload and download
     Buf<unsigned long long> chk;
@@ -384,6 +386,9 @@ SqDev sq_dev(gb2_sq_ctx *c)
     D.mu = c->mu;
     D.cnt = c->counters.p;
     D.dflag = c->dflag.p;
+    D.dstop = c->queued ? c->dstop.p : nullptr;
+    D.step = c->step;
+    D.hstop = c->h_pin + 4;
     D.mlp = c->mlp_on ? c->mlp.p : nullptr;
     return D;
 }
@@ -484,7 +489,7 @@ int sq_build(gb2_sq_ctx *c, bool transfer)
     SQCK(c->pti.alloc(ns));
     SQCK(c->ptj.alloc(ns));
     SQCK(c->work.alloc(2 * ns + 4));
-    SQCK(c->kind.alloc(ns));
+    SQCK(cudaMemsetAsync(c->work.p + 2 * ns, 0, 4 * sizeof(int), c->st));   // empty lists
     SQCK(c->rslot.alloc(ns));
     D = sq_dev(c);
     k_sq_neigh<<<nb(n), kB, 0, c->st>>>(D, G, c->cell_start.p, c->cell_atoms.p, nullptr, c->nbr.p, c->own.p, 1);
@@ -522,30 +527,19 @@ int sq_build(gb2_sq_ctx *c, bool transfer)
 }
 
 // the pair pass in work lists (screen, then the solves of the first contacts
-// and the warm starts), then the per-particle sums
-int sq_force(gb2_sq_ctx *c, int shearupdate)
+// and the warm starts), then the particles' sums and, on a step, the rest of
+// it (integrate) with the start of the next one (next)
+int sq_force(gb2_sq_ctx *c, int shearupdate, int integrate, int next)
 {
     SqDev D = sq_dev(c);
+    const size_t ns = (size_t)std::max<long>(c->nslots, 1);
+    SqWork W;
+    for (int l = 0; l < 2; l++) W.list[l] = c->work.p + l * ns;
+    W.n = c->work.p + 2 * ns;
+    W.next = W.n + 2;
     if (c->nslots > 0) {
-        const size_t ns = (size_t)c->nslots;
-        SqWork W;
-        for (int l = 0; l < 2; l++) W.list[l] = c->work.p + l * ns;
-        W.n = c->work.p + 2 * ns;
-        W.next = W.n + 2;
-        SQCK(cudaMemsetAsync(W.n, 0, 4 * sizeof(int), c->st));
-        k_sq_screen<<<nb(c->nslots), kB, 0, c->st>>>(D, c->own.p, (int)c->nslots, c->kind.p);
+        k_sq_screen<<<nb(c->nslots), kB, 0, c->st>>>(D, c->own.p, (int)c->nslots, W);
         SQCKL();
-        // the two work lists in slot order (stable selections; the counts
-        // stay on the device for the solve kernel)
-        thrust::counting_iterator<int> slots(0);
-        size_t bytes = 0;
-        cub::DeviceSelect::If(nullptr, bytes, slots, W.list[0], W.n, (int)ns, SlotKindIs{c->kind.p, 0}, c->st);
-        SQCK(c->tmp.alloc(bytes));
-        for (int l = 0; l < 2; l++) {
-            bytes = c->tmp.n;
-            SQCK(cub::DeviceSelect::If(c->tmp.p, bytes, slots, W.list[l], W.n + l, (int)ns,
-                                       SlotKindIs{c->kind.p, (signed char)l}, c->st));
-        }
         const float4 *guess = nullptr;
         if (D.mlp) {   // the learned guesses of the first contacts, one block per SM at most
             SQCK(c->guess.alloc(ns));
@@ -559,7 +553,7 @@ int sq_force(gb2_sq_ctx *c, int shearupdate)
         k_sq_solve<<<3 * c->nsm, kB, 0, c->st>>>(D, W, c->own.p, shearupdate, guess);
         SQCKL();
     }
-    k_sq_sum<<<nb(c->n), kB, 0, c->st>>>(D);
+    k_sq_advance<<<nb(std::max(c->n, 3)), kB, 0, c->st>>>(D, W, integrate, next);
     SQCKL();
     return 0;
 }
@@ -588,7 +582,10 @@ int gb2_sq_create(const gb2_sq_params *p, gb2_sq_ctx **out)
     c->mu = p->friction;
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
         pinned_slot_get(&c->h_pin) != 0 || c->counters.alloc(8) != cudaSuccess ||
-        c->dflag.alloc(1) != cudaSuccess ||
+        c->dflag.alloc(1) != cudaSuccess || c->dstop.alloc(1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->qev[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->qev[1], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->qev[2], cudaEventDisableTiming) != cudaSuccess ||
         cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->st) != cudaSuccess ||
         cudaEventCreate(&c->e0) != cudaSuccess || cudaEventCreate(&c->e1) != cudaSuccess) {
         pinned_slot_put(c->h_pin);
@@ -605,6 +602,8 @@ int gb2_sq_destroy(gb2_sq_ctx *c)
     if (!c) return 0;
     cudaStreamSynchronize(c->st);
     pinned_slot_put(c->h_pin);
+    for (cudaEvent_t e : c->qev)
+        if (e) cudaEventDestroy(e);
     if (c->e0) cudaEventDestroy(c->e0);
     if (c->e1) cudaEventDestroy(c->e1);
     cudaStream_t st = c->st;
@@ -676,7 +675,7 @@ int gb2_sq_setup(gb2_sq_ctx *c)
     SQCKL();
     int rc = sq_build(c, false);
     if (rc) return rc;
-    rc = sq_force(c, 0);
+    rc = sq_force(c, 0, 0, 0);
     if (rc) return rc;
     SQCK(cudaStreamSynchronize(c->st));
     c->setup_done = true;
@@ -687,22 +686,61 @@ int gb2_sq_run(gb2_sq_ctx *c, int nsteps)
 {
     if (!c) return GB2_ERR_ARG;
     if (!c->setup_done) return sq_err(c, GB2_ERR_STATE, "gb2_sq_setup must precede gb2_sq_run");
-    for (int s = 0; s < nsteps; s++) {
-        SQCK(cudaMemsetAsync(c->dflag.p, 0, sizeof(int), c->st));
-        SqDev D = sq_dev(c);
-        k_sq_initial<<<nb(c->n), kB, 0, c->st>>>(D, 1);
-        SQCKL();
-        SQCK(cudaMemcpyAsync(&c->h_pin[1], c->dflag.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    if (nsteps <= 0) {
         SQCK(cudaStreamSynchronize(c->st));
-        if (c->h_pin[1]) {
+        return 0;
+    }
+    // initial_integrate of the first step; every later one is part of the
+    // previous step's last kernel
+    SQCK(cudaMemsetAsync(c->dflag.p, 0, sizeof(int), c->st));
+    SqDev D0 = sq_dev(c);
+    k_sq_initial<<<nb(c->n), kB, 0, c->st>>>(D0);
+    SQCKL();
+    SQCK(cudaMemcpyAsync(&c->h_pin[1], c->dflag.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    SQCK(cudaStreamSynchronize(c->st));
+    bool rebuild = c->h_pin[1] != 0;
+    // Steps are queued ahead of the rebuild decision: the kernel that finds a
+    // displacement beyond skin/2 leaves its step in dstop and sets a
+    // page-locked word, and the kernels of later steps return at once.  The
+    // host looks at the word behind an event per step; once it is set it reads
+    // dstop behind everything queued and goes on from the step after it with a
+    // rebuild.  Waiting for the flag at every step left the device idle for a
+    // host round trip each time.
+    constexpr int kDepth = 3;
+    volatile int *hstop = c->h_pin + 4;
+    for (int s = 0; s < nsteps;) {
+        if (rebuild) {
             const int rc = sq_build(c, true);
             if (rc) return rc;
+            rebuild = false;
         }
-        int rc = sq_force(c, 1);
+        *hstop = 0;   // nothing in flight could set it
+        SQCK(cudaMemsetAsync(c->dstop.p, 0x7f, sizeof(int), c->st));
+        c->queued = true;
+        int head = s, launched = s, rc = 0;
+        while (!rc) {
+            while (!rc && launched < nsteps && launched - head < kDepth) {
+                c->step = launched;
+                rc = sq_force(c, 1, 1, launched < nsteps - 1);
+                if (!rc && cudaEventRecord(c->qev[launched % kDepth], c->st) != cudaSuccess)
+                    rc = sq_err(c, GB2_ERR_CUDA, "cudaEventRecord");
+                launched++;
+            }
+            if (rc || head == launched) break;
+            if (cudaEventSynchronize(c->qev[head % kDepth]) != cudaSuccess)
+                rc = sq_err(c, GB2_ERR_CUDA, "superquadric step: %s", cudaGetErrorString(cudaGetLastError()));
+            else if (*hstop != 0)
+                break;
+            else
+                head++;
+        }
+        c->queued = false;
         if (rc) return rc;
-        D = sq_dev(c);
-        k_sq_final<<<nb(c->n), kB, 0, c->st>>>(D);
-        SQCKL();
+        if (head == launched) break;   // every step is done
+        SQCK(cudaMemcpyAsync(&c->h_pin[5], c->dstop.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+        SQCK(cudaStreamSynchronize(c->st));
+        s = c->h_pin[5] + 1;   // the steps after dstop did nothing
+        rebuild = true;
     }
     SQCK(cudaStreamSynchronize(c->st));
     return 0;

@@ -473,23 +473,59 @@ __device__ __forceinline__ bool obb_intersect(const double *ca, const double *Ra
     return true;
 }
 
-// FixNVEAsphereBase, integration_scheme 1 helpers (src/math_extra.h, src/math_extra_liggghts_nonspherical.cpp:175)
+// FixNVEAsphereBase, integration_scheme 1 helpers (src/math_extra.h,
+// src/math_extra_liggghts_nonspherical.cpp:175).  Every product and sum is
+// rounded as written (no contraction), so the integrator does the reference's
+// arithmetic wherever it is inlined; its sincos is within an ulp of the host's.
+namespace integrator {
+
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
+// a += s b
+__device__ __forceinline__ void axpy(double s, double b, double &a) { a = add(a, mul(s, b)); }
+__device__ __forceinline__ double sum3(double a, double b, double c) { return add(add(a, b), c); }
+
+__device__ __forceinline__ void quat_to_mat(const double *q, double *m)
+{
+    const double w2 = mul(q[0], q[0]), i2 = mul(q[1], q[1]), j2 = mul(q[2], q[2]), k2 = mul(q[3], q[3]);
+    const double ti = 2.0 * q[1], tj = 2.0 * q[2], tk = 2.0 * q[3];
+    const double twoij = mul(ti, q[2]), twoik = mul(ti, q[3]), twojk = mul(tj, q[3]);
+    const double twoiw = mul(ti, q[0]), twojw = mul(tj, q[0]), twokw = mul(tk, q[0]);
+    m[0] = sub(sub(add(w2, i2), j2), k2);
+    m[1] = sub(twoij, twokw);
+    m[2] = add(twojw, twoik);
+    m[3] = add(twoij, twokw);
+    m[4] = sub(add(sub(w2, i2), j2), k2);
+    m[5] = sub(twojk, twoiw);
+    m[6] = sub(twoik, twojw);
+    m[7] = add(twojk, twoiw);
+    m[8] = add(sub(sub(w2, i2), j2), k2);
+}
+__device__ __forceinline__ void matvec(const double *m, const double *v, double *r)
+{
+    for (int k = 0; k < 3; k++) r[k] = sum3(mul(m[3 * k], v[0]), mul(m[3 * k + 1], v[1]), mul(m[3 * k + 2], v[2]));
+}
+__device__ __forceinline__ void tmatvec(const double *m, const double *v, double *r)
+{
+    for (int k = 0; k < 3; k++) r[k] = sum3(mul(m[k], v[0]), mul(m[3 + k], v[1]), mul(m[6 + k], v[2]));
+}
 __device__ __forceinline__ void quatvec(const double *a, const double *b, double *c)
 {
-    c[0] = -a[1] * b[0] - a[2] * b[1] - a[3] * b[2];
-    c[1] = a[0] * b[0] + a[2] * b[2] - a[3] * b[1];
-    c[2] = a[0] * b[1] + a[3] * b[0] - a[1] * b[2];
-    c[3] = a[0] * b[2] + a[1] * b[1] - a[2] * b[0];
+    c[0] = sub(sub(mul(-a[1], b[0]), mul(a[2], b[1])), mul(a[3], b[2]));
+    c[1] = sub(add(mul(a[0], b[0]), mul(a[2], b[2])), mul(a[3], b[1]));
+    c[2] = sub(add(mul(a[0], b[1]), mul(a[3], b[0])), mul(a[1], b[2]));
+    c[3] = sub(add(mul(a[0], b[2]), mul(a[1], b[1])), mul(a[2], b[0]));
 }
 __device__ __forceinline__ void invquatvec(const double *a, const double *b, double *c)
 {
-    c[0] = -a[1] * b[0] + a[0] * b[1] + a[3] * b[2] - a[2] * b[3];
-    c[1] = -a[2] * b[0] - a[3] * b[1] + a[0] * b[2] + a[1] * b[3];
-    c[2] = -a[3] * b[0] + a[2] * b[1] - a[1] * b[2] + a[0] * b[3];
+    c[0] = sub(add(add(mul(-a[1], b[0]), mul(a[0], b[1])), mul(a[3], b[2])), mul(a[2], b[3]));
+    c[1] = add(add(sub(mul(-a[2], b[0]), mul(a[3], b[1])), mul(a[0], b[2])), mul(a[1], b[3]));
+    c[2] = add(sub(add(mul(-a[3], b[0]), mul(a[2], b[1])), mul(a[1], b[2])), mul(a[0], b[3]));
 }
 __device__ __forceinline__ void no_squish_rotate(int k, double *p, double *q, const double *inertia, double dt)
 {
-    double kp[4] = {0, 0, 0, 0}, kq[4] = {0, 0, 0, 0};
+    double kp[4], kq[4];
     if (k == 1) {
         kq[0] = -q[1]; kp[0] = -p[1]; kq[1] = q[0]; kp[1] = p[0];
         kq[2] = q[3]; kp[2] = p[3]; kq[3] = -q[2]; kp[3] = -p[2];
@@ -500,17 +536,19 @@ __device__ __forceinline__ void no_squish_rotate(int k, double *p, double *q, co
         kq[0] = -q[3]; kp[0] = -p[3]; kq[1] = q[2]; kp[1] = p[2];
         kq[2] = -q[1]; kp[2] = -p[1]; kq[3] = q[0]; kp[3] = p[0];
     }
-    double phi = p[0] * kq[0] + p[1] * kq[1] + p[2] * kq[2] + p[3] * kq[3];
+    double phi = add(sum3(mul(p[0], kq[0]), mul(p[1], kq[1]), mul(p[2], kq[2])), mul(p[3], kq[3]));
     phi /= 4.0 * inertia[k - 1];
     double s_phi, c_phi;
-    sincos(dt * phi, &s_phi, &c_phi);
+    sincos(mul(dt, phi), &s_phi, &c_phi);
     for (int m = 0; m < 4; m++) {
-        const double pm = c_phi * p[m] + s_phi * kp[m];
-        const double qm = c_phi * q[m] + s_phi * kq[m];
+        const double pm = add(mul(c_phi, p[m]), mul(s_phi, kp[m]));
+        const double qm = add(mul(c_phi, q[m]), mul(s_phi, kq[m]));
         p[m] = pm;
         q[m] = qm;
     }
 }
+
+}  // namespace integrator
 
 }  // namespace sq
 }  // namespace gb2

@@ -34,95 +34,128 @@ struct SqDev {
     // counters: iterations, solves, pairs solved, learned guesses used, learned guesses rejected
     unsigned long long *cnt;
     int *dflag;
+    // steps queued ahead: the lowest step whose end asked for a rebuild of the
+    // next one (null when not queuing), this launch's step, and a page-locked
+    // host word set with it
+    int *dstop;
+    int step;
+    volatile int *hstop;
     // learned initial guess (null when off)
     const float *mlp;
 };
 
+// One particle's state through the integrator
+struct SqBody {
+    dbl4 x, v;
+    double q[4], L[3], w[3];
+};
+
+__device__ __forceinline__ bool sq_cancelled(const SqDev &D) { return D.dstop && *(volatile int *)D.dstop < D.step; }
+
 // FixNVEAsphereBase::initial_integrate, integration_scheme 1
-// (src/fix_nve_asphere_base.cpp:319-444), and Neighbor::check_distance
-__global__ void k_sq_initial(SqDev D, int check)
+// (src/fix_nve_asphere_base.cpp:319-444) with force f and torque tq
+__device__ __forceinline__ void sq_initial(const SqDev &D, SqBody &B, const dbl4 &f, const dbl4 &tq, const dbl4 &in4)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= D.n) return;
     const double dtv = D.dt, dtf = 0.5 * D.dt * 1.0, dtf2 = 2.0 * dtf, dtq = 0.5 * dtv;
-    dbl4 x = D.x[i], v = D.v[i], q4 = D.q[i];
-    const dbl4 f = D.f[i], tq = D.t[i], in4 = D.inert[i], L4 = D.L[i];
-    double q[4] = {q4.x, q4.y, q4.z, q4.w};
+    using namespace integrator;
     const double in[3] = {in4.x, in4.y, in4.z};
     double R[9], mbody[3], conjqm[4], tbody[3], fquat[4], wbody[3];
-    quat_to_mat(q, R);
-    const double dtfm = dtf / v.w;
-    v.x += dtfm * f.x;
-    v.y += dtfm * f.y;
-    v.z += dtfm * f.z;
-    x.x += dtv * v.x;
-    x.y += dtv * v.y;
-    x.z += dtv * v.z;
-    const double Lv[3] = {L4.x, L4.y, L4.z}, Tv[3] = {tq.x, tq.y, tq.z};
-    tmatvec(R, Lv, mbody);
-    quatvec(q, mbody, conjqm);
+    integrator::quat_to_mat(B.q, R);
+    const double dtfm = dtf / B.v.w;
+    axpy(dtfm, f.x, B.v.x);
+    axpy(dtfm, f.y, B.v.y);
+    axpy(dtfm, f.z, B.v.z);
+    axpy(dtv, B.v.x, B.x.x);
+    axpy(dtv, B.v.y, B.x.y);
+    axpy(dtv, B.v.z, B.x.z);
+    const double Tv[3] = {tq.x, tq.y, tq.z};
+    integrator::tmatvec(R, B.L, mbody);
+    quatvec(B.q, mbody, conjqm);
     for (int k = 0; k < 4; k++) conjqm[k] *= 2.0;
-    tmatvec(R, Tv, tbody);
-    quatvec(q, tbody, fquat);
-    for (int k = 0; k < 4; k++) conjqm[k] += dtf2 * fquat[k];
-    no_squish_rotate(3, conjqm, q, in, dtq);
-    no_squish_rotate(2, conjqm, q, in, dtq);
-    no_squish_rotate(1, conjqm, q, in, dtv);
-    no_squish_rotate(2, conjqm, q, in, dtq);
-    no_squish_rotate(3, conjqm, q, in, dtq);
-    const double norm = 1.0 / sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
-    for (int k = 0; k < 4; k++) q[k] *= norm;
-    quat_to_mat(q, R);
-    invquatvec(q, conjqm, mbody);
+    integrator::tmatvec(R, Tv, tbody);
+    quatvec(B.q, tbody, fquat);
+    for (int k = 0; k < 4; k++) axpy(dtf2, fquat[k], conjqm[k]);
+    no_squish_rotate(3, conjqm, B.q, in, dtq);
+    no_squish_rotate(2, conjqm, B.q, in, dtq);
+    no_squish_rotate(1, conjqm, B.q, in, dtv);
+    no_squish_rotate(2, conjqm, B.q, in, dtq);
+    no_squish_rotate(3, conjqm, B.q, in, dtq);
+    const double norm =
+        1.0 / sqrt(add(sum3(mul(B.q[0], B.q[0]), mul(B.q[1], B.q[1]), mul(B.q[2], B.q[2])), mul(B.q[3], B.q[3])));
+    for (int k = 0; k < 4; k++) B.q[k] *= norm;
+    integrator::quat_to_mat(B.q, R);
+    invquatvec(B.q, conjqm, mbody);
     for (int d = 0; d < 3; d++) mbody[d] *= 0.5;
     for (int d = 0; d < 3; d++) wbody[d] = mbody[d] / in[d];
-    double Lo[3], wo[3];
-    matvec(R, mbody, Lo);
-    matvec(R, wbody, wo);
-    D.x[i] = x;
-    D.v[i] = v;
-    D.q[i] = dbl4{q[0], q[1], q[2], q[3]};
-    D.L[i] = dbl4{Lo[0], Lo[1], Lo[2], 0.0};
-    D.w[i] = dbl4{wo[0], wo[1], wo[2], 0.0};
-    if (check) {
-        const dbl4 h = D.xhold[i];
-        const double dx = x.x - h.x, dy = x.y - h.y, dz = x.z - h.z;
-        if (dx * dx + dy * dy + dz * dz > D.triggersq) *D.dflag = 1;
-    }
+    integrator::matvec(R, mbody, B.L);
+    integrator::matvec(R, wbody, B.w);
 }
 
 // FixNVEAsphereBase::final_integrate, integration_scheme 1 (:523-620)
-__global__ void k_sq_final(SqDev D)
+__device__ __forceinline__ void sq_final(const SqDev &D, SqBody &B, const dbl4 &f, const dbl4 &tq, const dbl4 &in4)
+{
+    const double dtf = 0.5 * D.dt * 1.0, dtf2 = dtf * 2.0;
+    using namespace integrator;
+    const double in[3] = {in4.x, in4.y, in4.z};
+    double R[9], tbody[3], mbody[3], conjqm[4], fquat[4], wbody[3];
+    const double dtfm = dtf / B.v.w;
+    integrator::quat_to_mat(B.q, R);
+    axpy(dtfm, f.x, B.v.x);
+    axpy(dtfm, f.y, B.v.y);
+    axpy(dtfm, f.z, B.v.z);
+    const double Tv[3] = {tq.x, tq.y, tq.z};
+    integrator::tmatvec(R, Tv, tbody);
+    integrator::tmatvec(R, B.L, mbody);
+    quatvec(B.q, mbody, conjqm);
+    for (int k = 0; k < 4; k++) conjqm[k] *= 2.0;
+    quatvec(B.q, tbody, fquat);
+    for (int k = 0; k < 4; k++) axpy(dtf2, fquat[k], conjqm[k]);
+    invquatvec(B.q, conjqm, mbody);
+    for (int d = 0; d < 3; d++) mbody[d] *= 0.5;
+    for (int d = 0; d < 3; d++) wbody[d] = mbody[d] / in[d];
+    integrator::matvec(R, mbody, B.L);
+    integrator::matvec(R, wbody, B.w);
+}
+
+__device__ __forceinline__ SqBody sq_load(const SqDev &D, int i)
+{
+    SqBody B;
+    B.x = D.x[i];
+    B.v = D.v[i];
+    const dbl4 q = D.q[i], L = D.L[i];
+    B.q[0] = q.x, B.q[1] = q.y, B.q[2] = q.z, B.q[3] = q.w;
+    B.L[0] = L.x, B.L[1] = L.y, B.L[2] = L.z;
+    return B;
+}
+
+__device__ __forceinline__ void sq_store(const SqDev &D, int i, const SqBody &B, bool moved)
+{
+    if (moved) {
+        D.x[i] = B.x;
+        D.q[i] = dbl4{B.q[0], B.q[1], B.q[2], B.q[3]};
+    }
+    D.v[i] = B.v;
+    D.L[i] = dbl4{B.L[0], B.L[1], B.L[2], 0.0};
+    D.w[i] = dbl4{B.w[0], B.w[1], B.w[2], 0.0};
+}
+
+// Neighbor::check_distance
+__device__ __forceinline__ bool sq_far(const SqDev &D, int i, const dbl4 &x)
+{
+    const dbl4 h = D.xhold[i];
+    const double dx = x.x - h.x, dy = x.y - h.y, dz = x.z - h.z;
+    return dx * dx + dy * dy + dz * dz > D.triggersq;
+}
+
+// the first step of a run: initial_integrate and the displacement test
+__global__ void k_sq_initial(SqDev D)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= D.n) return;
-    const double dtf = 0.5 * D.dt * 1.0, dtf2 = dtf * 2.0;
-    dbl4 v = D.v[i];
-    const dbl4 q4 = D.q[i], f = D.f[i], tq = D.t[i], in4 = D.inert[i], L4 = D.L[i];
-    const double q[4] = {q4.x, q4.y, q4.z, q4.w};
-    const double in[3] = {in4.x, in4.y, in4.z};
-    double R[9], tbody[3], mbody[3], conjqm[4], fquat[4], wbody[3];
-    const double dtfm = dtf / v.w;
-    quat_to_mat(q, R);
-    v.x += dtfm * f.x;
-    v.y += dtfm * f.y;
-    v.z += dtfm * f.z;
-    const double Tv[3] = {tq.x, tq.y, tq.z}, Lv[3] = {L4.x, L4.y, L4.z};
-    tmatvec(R, Tv, tbody);
-    tmatvec(R, Lv, mbody);
-    quatvec(q, mbody, conjqm);
-    for (int k = 0; k < 4; k++) conjqm[k] *= 2.0;
-    quatvec(q, tbody, fquat);
-    for (int k = 0; k < 4; k++) conjqm[k] += dtf2 * fquat[k];
-    invquatvec(q, conjqm, mbody);
-    for (int d = 0; d < 3; d++) mbody[d] *= 0.5;
-    for (int d = 0; d < 3; d++) wbody[d] = mbody[d] / in[d];
-    double Lo[3], wo[3];
-    matvec(R, mbody, Lo);
-    matvec(R, wbody, wo);
-    D.v[i] = v;
-    D.L[i] = dbl4{Lo[0], Lo[1], Lo[2], 0.0};
-    D.w[i] = dbl4{wo[0], wo[1], wo[2], 0.0};
+    SqBody B = sq_load(D, i);
+    sq_initial(D, B, D.f[i], D.t[i], D.inert[i]);
+    sq_store(D, i, B, true);
+    if (sq_far(D, i, B.x)) *D.dflag = 1;
 }
 
 // omega from angular momentum (set-up)
@@ -341,8 +374,8 @@ __device__ __forceinline__ void first_contact(const float *out, const double *ci
 // src/pair_gran_base.h:255-430, src/surface_model_superquadric.h:108-205,
 // non-spherical Hertz/history): k_sq_screen tests every half-list slot
 // (bounding spheres, oriented boxes) and marks the slots that need a
-// contact-point solve for one of two lists, first contacts and warm starts
-// (a previous point exists), which stable selections gather in slot order;
+// contact-point solve on one of two lists, first contacts and warm starts
+// (a previous point exists);
 // k_sq_solve (gb2_sq_solve.cuh) runs the solves, first contacts first: their
 // chains, through the homotopy or the learned guess, are the longest, so they
 // start at once and the short warm starts fill the GPU around them.  Every
@@ -352,23 +385,18 @@ __device__ __forceinline__ void first_contact(const float *out, const double *ci
 // lists of one pair pass: 0 first contacts, 1 warm starts
 struct SqWork {
     int *list[2];
-    int *n;      // item counts, [2]
+    int *n;      // item counts, [2]; zeroed by the step's end (k_sq_advance)
     int *next;   // items taken (over both lists)
-};
-
-// the work list a screened slot joins: 0 first contact, 1 warm start, -1 none
-struct SlotKindIs {
-    const signed char *kind;
-    signed char want;
-    __host__ __device__ bool operator()(int sl) const { return kind[sl] == want; }
 };
 
 // every slot: no force unless a solve below finds a contact; the bounding
 // spheres and (for a pair not yet intersecting) the oriented boxes decide
-// whether the slot needs a solve and which kind (kind[sl]; the host gathers
-// the work lists from it in slot order, so they are the same in every run)
-__global__ void k_sq_screen(SqDev D, const int *__restrict__ own, int nslots, signed char *kind_out)
+// whether the slot needs a solve and which kind, and a warp appends its slots
+// to the two lists with one atomic each (the order of a list affects no
+// result; two stable selections were four launches, ~15 us of a step)
+__global__ void k_sq_screen(SqDev D, const int *__restrict__ own, int nslots, SqWork W)
 {
+    if (sq_cancelled(D)) return;
     const int sl = blockIdx.x * blockDim.x + threadIdx.x;
     int kind = -1;
     if (sl < nslots) {
@@ -396,15 +424,22 @@ __global__ void k_sq_screen(SqDev D, const int *__restrict__ own, int nslots, si
             else kind = state == FAR ? 0 : 1;
         }
     }
-    if (sl < nslots) kind_out[sl] = (signed char)kind;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+        const unsigned m = __ballot_sync(0xffffffffu, kind == l);
+        if (!m) continue;
+        int base = 0;
+        if (lane == __ffs(m) - 1) base = atomicAdd(&W.n[l], __popc(m));
+        base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
+        if (kind == l) W.list[l][base + __popc(m & ((1u << lane) - 1u))] = sl;
+    }
 }
 
 // per-atom sums in the reference's order: slots where the atom is the j
 // side (ascending i), then its own slots
-__global__ void k_sq_sum(SqDev D)
+__device__ __forceinline__ void sq_sums(const SqDev &D, int k, dbl4 &Fo, dbl4 &To)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= D.n) return;
     double F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
     for (int r = D.rstart[k]; r < D.rstart[k + 1]; r++) {
         const int sl = D.rslot[r];
@@ -429,8 +464,40 @@ __global__ void k_sq_sum(SqDev D)
         T[1] += t.y;
         T[2] += t.z;
     }
-    D.f[k] = dbl4{F[0], F[1], F[2], 0.0};
-    D.t[k] = dbl4{T[0], T[1], T[2], 0.0};
+    Fo = dbl4{F[0], F[1], F[2], 0.0};
+    To = dbl4{T[0], T[1], T[2], 0.0};
+}
+
+// The end of a pair pass: the sums and, on a step (integrate), final_integrate
+// and -- when the run continues (next) -- the next step's initial_integrate
+// with its displacement test, per particle in one kernel: three kernels each
+// read and wrote the same records.  Leaves the work lists empty for the next
+// pass.
+__global__ void k_sq_advance(SqDev D, SqWork W, int integrate, int next)
+{
+    if (sq_cancelled(D)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 3) W.n[i] = 0;   // n[2] and next, which follows them
+    if (i >= D.n) return;
+    dbl4 f, t;
+    sq_sums(D, i, f, t);
+    D.f[i] = f;
+    D.t[i] = t;
+    if (!integrate) return;
+    const dbl4 in4 = D.inert[i];
+    SqBody B = sq_load(D, i);
+    sq_final(D, B, f, t, in4);
+    if (next) {
+        sq_initial(D, B, f, t, in4);
+        if (sq_far(D, i, B.x)) {
+            *D.dflag = 1;
+            if (D.dstop) {
+                atomicMin(D.dstop, D.step);
+                *D.hstop = 1;
+            }
+        }
+    }
+    sq_store(D, i, B, next != 0);
 }
 
 }  // namespace sq
