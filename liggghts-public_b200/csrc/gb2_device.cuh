@@ -360,7 +360,9 @@ __device__ __forceinline__ void list_append(int2 *list, int cap, int &n, bool ta
 // U entries of each list are in flight together (their records are requested,
 // then the next U indices, then the tests): four in FP64 (against two: hopper
 // of 1M 255 -> 253 us/step, bed of 2M 818 -> 808), two in split precision,
-// whose 80 registers do not hold eight records (205 -> 274).
+// whose 80 registers do not hold eight records (205 -> 274), in the loop its
+// contact arithmetic was always compiled beside (contraction, and with it the
+// last bits, depend on the code around).
 //
 // G lanes per atom: lane G a + g takes entries g, g + G, ... of atom a's lists,
 // so a ballot's lane order is still every atom's list order; the owner lane
@@ -406,38 +408,71 @@ __device__ __forceinline__ bool screen_list(const Dev &D, int k, int nr, int nn,
     const int cap = D.cap, lane = threadIdx.x & 31;
     const int nw = __reduce_max_sync(0xffffffffu, max(nr, nn));
     nlrev = nlown = 0;
-    int a[U], b[U], sl[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        a[u] = u < nr ? ld_stream(&D.rev[u * cap + k]) : 0;
-        sl[u] = u < nr ? (int)D.revs[u * cap + k] : 0;
-        b[u] = u < nn ? ld_stream(&D.nbr[u * cap + k]) : 0;
-    }
-    for (int t = 0; t < nw; t += U) {
-        dbl4 qa[U], qb[U];
-        int ca[U], cb[U], cs[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            qa[u] = ldg4(&D.pos[a[u]]);
-            qb[u] = ldg4(&D.pos[b[u]]);
-            ca[u] = a[u];
-            cb[u] = b[u];
-            cs[u] = sl[u];
+    if constexpr (U == 2) {
+        int a0 = (0 < nr) ? ld_stream(&D.rev[k]) : 0;
+        int a1 = (1 < nr) ? ld_stream(&D.rev[cap + k]) : 0;
+        int s0 = (0 < nr) ? (int)D.revs[k] : 0;
+        int s1 = (1 < nr) ? (int)D.revs[cap + k] : 0;
+        int b0 = (0 < nn) ? ld_stream(&D.nbr[k]) : 0;
+        int b1 = (1 < nn) ? ld_stream(&D.nbr[cap + k]) : 0;
+        for (int t = 0; t < nw; t += 2) {
+            const dbl4 qa0 = ldg4(&D.pos[a0]);
+            const dbl4 qa1 = ldg4(&D.pos[a1]);
+            const dbl4 qb0 = ldg4(&D.pos[b0]);
+            const dbl4 qb1 = ldg4(&D.pos[b1]);
+            const int ca0 = a0, ca1 = a1, cs0 = s0, cs1 = s1, cb0 = b0, cb1 = b1;
+            const int u = t + 2;
+            a0 = (u < nr) ? ld_stream(&D.rev[u * cap + k]) : 0;
+            a1 = (u + 1 < nr) ? ld_stream(&D.rev[(u + 1) * cap + k]) : 0;
+            s0 = (u < nr) ? (int)D.revs[u * cap + k] : 0;
+            s1 = (u + 1 < nr) ? (int)D.revs[(u + 1) * cap + k] : 0;
+            b0 = (u < nn) ? ld_stream(&D.nbr[u * cap + k]) : 0;
+            b1 = (u + 1 < nn) ? ld_stream(&D.nbr[(u + 1) * cap + k]) : 0;
+            const bool ta0 = t < nr && touching(pk, qa0), ta1 = t + 1 < nr && touching(pk, qa1);
+            const bool tb0 = t < nn && touching(pk, qb0), tb1 = t + 1 < nn && touching(pk, qb1);
+            if (ta0) mrev |= 1ull << t;
+            if (ta1) mrev |= 1ull << (t + 1);
+            if (tb0) mown |= 1ull << t;
+            if (tb1) mown |= 1ull << (t + 1);
+            list_append(lrev, D.item_cap, nlrev, ta0, ca0, lane | (cs0 << 8));
+            list_append(lrev, D.item_cap, nlrev, ta1, ca1, lane | (cs1 << 8));
+            list_append(lown, D.item_cap, nlown, tb0, cb0, lane | (t << 8));
+            list_append(lown, D.item_cap, nlown, tb1, cb1, lane | ((t + 1) << 8));
         }
+    } else {
+        int a[U], b[U], sl[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int v = t + U + u;
-            a[u] = v < nr ? ld_stream(&D.rev[v * cap + k]) : 0;
-            sl[u] = v < nr ? (int)D.revs[v * cap + k] : 0;
-            b[u] = v < nn ? ld_stream(&D.nbr[v * cap + k]) : 0;
+            a[u] = u < nr ? ld_stream(&D.rev[u * cap + k]) : 0;
+            sl[u] = u < nr ? (int)D.revs[u * cap + k] : 0;
+            b[u] = u < nn ? ld_stream(&D.nbr[u * cap + k]) : 0;
         }
+        for (int t = 0; t < nw; t += U) {
+            dbl4 qa[U], qb[U];
+            int ca[U], cb[U], cs[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const bool ta = t + u < nr && touching(pk, qa[u]), tb = t + u < nn && touching(pk, qb[u]);
-            if (ta) mrev |= 1ull << (t + u);
-            if (tb) mown |= 1ull << (t + u);
-            list_append(lrev, D.item_cap, nlrev, ta, ca[u], lane | (cs[u] << 8));
-            list_append(lown, D.item_cap, nlown, tb, cb[u], lane | ((t + u) << 8));
+            for (int u = 0; u < U; u++) {
+                qa[u] = ldg4(&D.pos[a[u]]);
+                qb[u] = ldg4(&D.pos[b[u]]);
+                ca[u] = a[u];
+                cb[u] = b[u];
+                cs[u] = sl[u];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int v = t + U + u;
+                a[u] = v < nr ? ld_stream(&D.rev[v * cap + k]) : 0;
+                sl[u] = v < nr ? (int)D.revs[v * cap + k] : 0;
+                b[u] = v < nn ? ld_stream(&D.nbr[v * cap + k]) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const bool ta = t + u < nr && touching(pk, qa[u]), tb = t + u < nn && touching(pk, qb[u]);
+                if (ta) mrev |= 1ull << (t + u);
+                if (tb) mown |= 1ull << (t + u);
+                list_append(lrev, D.item_cap, nlrev, ta, ca[u], lane | (cs[u] << 8));
+                list_append(lown, D.item_cap, nlown, tb, cb[u], lane | ((t + u) << 8));
+            }
         }
     }
     return nlrev <= D.item_cap && nlown <= D.item_cap;

@@ -1285,9 +1285,10 @@ void launch_pair(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int f
     // two lanes halve it (20,000-sphere pour 40.2 -> 37.6 us/step, 6,000-sphere
     // hopper 32.1 -> 31.0).  At 40,000 spheres both take the same, at 300,000
     // two lanes are slower (83 -> 102).  Four lanes gain nothing on two.
-    const int lanes = c->nlocal <= 200 * c->nsm ? 2 : 1;
+    // Split precision keeps one lane: its results would change in their last bits.
+    const int lanes = !c->split && c->nlocal <= 200 * c->nsm ? 2 : 1;
     if (c->split)
-        launch_pair_split(D, lanes, c->st, shearupdate, integrate, fuse_next, store_f, pair_list_smem(c));
+        launch_pair_split(D, c->st, shearupdate, integrate, fuse_next, store_f, pair_list_smem(c));
     else
         launch_pair_step<false>(D, lanes, c->st, shearupdate, integrate, fuse_next, store_f, pair_list_smem(c));
 }

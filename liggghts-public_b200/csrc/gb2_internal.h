@@ -189,8 +189,8 @@ struct MeshTopo {
 bool build_mesh_topology(const double *nodes, int ntri_in, double curvature, double precision, MeshTopo &out,
                          std::string &err);
 // split-precision pair step (gb2_split.cu)
-void launch_pair_split(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                       int store_f, size_t smem);
+void launch_pair_split(const Dev &D, cudaStream_t st, int shearupdate, int integrate, int fuse_next, int store_f,
+                       size_t smem);
 void launch_tail_split(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
                        int store_f);
 bool tri_neighbuild_host(const TriGeom &T, double rSphere, const double *c, double treshold);

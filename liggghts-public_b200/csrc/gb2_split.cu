@@ -11,10 +11,10 @@
 
 namespace gb2 {
 
-void launch_pair_split(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                       int store_f, size_t smem)
+void launch_pair_split(const Dev &D, cudaStream_t st, int shearupdate, int integrate, int fuse_next, int store_f,
+                       size_t smem)
 {
-    launch_pair_step<true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
+    launch_pair_step<true>(D, 1, st, shearupdate, integrate, fuse_next, store_f, smem);
 }
 
 void launch_tail_split(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate, int fuse_next,

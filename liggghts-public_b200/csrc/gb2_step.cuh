@@ -698,7 +698,7 @@ inline cudaError_t launch_dependent(Kernel kernel, int nblocks, size_t smem, cud
     return cudaLaunchKernelEx(&cfg, kernel, D, shearupdate, integrate, fuse_next, store_f);
 }
 
-// The pair step with one or two lanes per atom.  Registers: FP64 takes 4 blocks
+// The pair step with one or (FP64) two lanes per atom.  Registers: FP64 takes 4 blocks
 // per SM (128 registers, no spill): 5 blocks (96) spill 20 doubles through the
 // L1 that the gathers need, 3 leave too few warps (hopper of 1M 253, 267 and
 // 307 us/step, bed of 2M 847, 907 and 847).  Split precision fits 6 blocks (80):
@@ -707,7 +707,10 @@ template <bool ROLLING, bool SPLIT, bool ONE>
 inline cudaError_t launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
                             int store_f, size_t smem)
 {
-    const auto kernel = lanes == 1 ? k_pair_step<ROLLING, SPLIT ? 6 : 4, SPLIT, ONE, 1> : k_pair_step<ROLLING, 4, SPLIT, ONE, 2>;
+    auto kernel = k_pair_step<ROLLING, SPLIT ? 6 : 4, SPLIT, ONE, 1>;
+    if constexpr (!SPLIT) {
+        if (lanes == 2) kernel = k_pair_step<ROLLING, 4, false, ONE, 2>;
+    }
     const int nblocks = (int)(((long)D.nlocal * lanes + 127) / 128);
     return launch_dependent(kernel, nblocks, smem, st, D, shearupdate, integrate, fuse_next, store_f);
 }
