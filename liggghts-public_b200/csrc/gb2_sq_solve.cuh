@@ -4,8 +4,12 @@
 // (lane 3 of each half adds zeros), so the six powers of a shape function
 // evaluation -- the arithmetic of a solve -- run side by side, one per lane,
 // and the value, gradient and Hessian sums are shuffles.  The scalars of the
-// solve are replicated in the eight lanes (the butterfly sums are the same
-// in every lane bit for bit), so control flow is uniform in a group.
+// solve are replicated in the eight lanes: the butterfly sums round every
+// product and every sum by itself, so they are the same in each lane bit for
+// bit.  Control flow is uniform in a group by construction: what a group does
+// next is decided by its first lane and taken from it by the others, so its
+// shuffles and barriers are reached by all eight lanes whatever the compiler
+// makes of the replicated arithmetic.
 //
 // What bounds it: a step holds few solves (27k among 1M slots of a 200k
 // packing) and the longest chain -- a first contact's homotopy, 11 stages and
@@ -87,16 +91,20 @@ __device__ __forceinline__ bool solve_bordered(const double *h, const double *c,
     return D != 0.0 && !isnan(D);
 }
 
-// the sum of v over the lanes of one body (4) or of the pair (8)
-__device__ __forceinline__ double sum4(unsigned mask, double v)
+// The sum of a * b over the lanes of one body (4) or of the pair (8), the same
+// bits in each of them.  Product and sums are rounded one by one: contracted,
+// a lane would add its own unrounded product to its partner's rounded one, and
+// the two lanes' sums would differ.
+__device__ __forceinline__ double sum4(unsigned mask, double a, double b)
 {
-    v += __shfl_xor_sync(mask, v, 1);
-    return v + __shfl_xor_sync(mask, v, 2);
+    double v = __dmul_rn(a, b);
+    v = __dadd_rn(v, __shfl_xor_sync(mask, v, 1));
+    return __dadd_rn(v, __shfl_xor_sync(mask, v, 2));
 }
-__device__ __forceinline__ double sum8(unsigned mask, double v)
+__device__ __forceinline__ double sum8(unsigned mask, double a, double b)
 {
-    v = sum4(mask, v);
-    return v + __shfl_xor_sync(mask, v, 4);
+    const double v = sum4(mask, a, b);
+    return __dadd_rn(v, __shfl_xor_sync(mask, v, 4));
 }
 
 // one lane's share of a body: its axis
@@ -257,11 +265,11 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
         const double ka = X.koef * X.inv;
         const double g0 = ka * X.n * sgn(u) * p1;
         const double dnew = ka * (X.n * (X.n - 1.0) * p2) * X.inv;
-        const double f_own = X.koef * (sum4(FULL, p1 * au) - 1.0);
+        const double f_own = X.koef * (sum4(FULL, p1, au) - 1.0);
         double go[3];
-        go[0] = sum4(FULL, line ? g0 * dl : X.rc[0] * g0);
-        go[1] = sum4(FULL, X.rc[1] * g0);
-        go[2] = sum4(FULL, X.rc[2] * g0);
+        go[0] = sum4(FULL, line ? dl : X.rc[0], g0);
+        go[1] = sum4(FULL, X.rc[1], g0);
+        go[2] = sum4(FULL, X.rc[2], g0);
         double tA[3], tB[3];
         for (int k = 0; k < 3; k++) {
             const double gx = __shfl_xor_sync(FULL, go[k], 4);
@@ -378,14 +386,14 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
         // ---- Newton steps (all lanes take part in the sums; the groups that asked use the result)
         if (__any_sync(FULL, step)) {
             const double w = second ? mu * mu * dcur : dcur;
-            const double r0 = X.rc[0] * w, r1 = X.rc[1] * w;
+            const double r0 = X.rc[0] * w, r1 = X.rc[1] * w, r2 = X.rc[2] * w;
             double h[6], cc[3], dd[3];
-            h[0] = sum8(FULL, r0 * X.rc[0]);
-            h[1] = sum8(FULL, r0 * X.rc[1]);
-            h[2] = sum8(FULL, r0 * X.rc[2]);
-            h[3] = sum8(FULL, r1 * X.rc[1]);
-            h[4] = sum8(FULL, r1 * X.rc[2]);
-            h[5] = sum8(FULL, X.rc[2] * w * X.rc[2]);
+            h[0] = sum8(FULL, r0, X.rc[0]);
+            h[1] = sum8(FULL, r0, X.rc[1]);
+            h[2] = sum8(FULL, r0, X.rc[2]);
+            h[3] = sum8(FULL, r1, X.rc[1]);
+            h[4] = sum8(FULL, r1, X.rc[2]);
+            h[5] = sum8(FULL, r2, X.rc[2]);
             for (int k = 0; k < 3; k++) {
                 cc[k] = 2.0 * mu * gB[k];
                 dd[k] = gA[k] - gB[k];
@@ -414,13 +422,21 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
             }
         }
 
+        // the first lane's decision for the group
+        const int decided = __shfl_sync(FULL, state | (end ? 16 : 0), lane & 24);
+        state = decided & 15;
+        end = (decided & 16) != 0;
+
         // ---- the end of one solve: the next stage, the homotopy after a
         // rejected guess, or the item's result
         if (end) {
             c_it += it;
             c_sv++;
             it = 0;
-            const bool rejected = phase == 0 && (fail || !(merit1 < 1e-10));
+            const unsigned verdict =
+                __shfl_sync(gmask, (phase == 0 && (fail || !(merit1 < 1e-10)) ? 1u : 0u) |
+                                       (fmax(fi, fj) < 0.0 ? 2u : 0u), lane & 24);
+            const bool rejected = verdict & 1u, overlap = verdict & 2u;
             fail = false;
             if (rejected || (phase == 1 && stage < nstage)) {
                 if (rejected) {
@@ -445,7 +461,7 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
                 if (used == 1) c_used++;
                 if (used == -1) c_rej++;
                 if (gl == 0) D.cp[sl] = dbl4{pt[0], pt[1], pt[2], 0.0};
-                if (!(fmax(fi, fj) < 0.0)) {
+                if (!overlap) {
                     if (gl == 0) D.state[sl] = CLOSE;
                     state = Q_IDLE;
                 } else {   // the overlap along the normal: a line search per body
@@ -469,8 +485,8 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
                     smin = fmin(smin, __shfl_xor_sync(gmask, smin, 1));
                     smin = fmin(smin, __shfl_xor_sync(gmask, smin, 2));
                     const double x0 = lx * X.inv, nx = dl * X.inv;
-                    const double qa = sum4(gmask, nx * nx), qb = 2.0 * sum4(gmask, x0 * nx);
-                    const double qc = sum4(gmask, x0 * x0) - 1.0;
+                    const double qa = sum4(gmask, nx, nx), qb = 2.0 * sum4(gmask, x0, nx);
+                    const double qc = sum4(gmask, x0, x0) - 1.0;
                     ldone = false;
                     if (comp_double(X.n, 2.0, 1e-2)) {   // an ellipsoid: the quadratic
                         const double eps0 = 1e-14;
@@ -549,6 +565,7 @@ __global__ void __launch_bounds__(128, 3) k_sq_solve(SqDev D, SqWork W, const in
         __syncwarp();
 
         // ---- both lines done: contact forces (non-spherical kinematics, Hertz, tangential history)
+        ldone = __shfl_sync(FULL, (int)ldone, lane & 28) != 0;   // each body's first lane decides for it
         const bool both = __shfl_xor_sync(FULL, (int)ldone, 4) != 0 && ldone;
         const double aother = __shfl_xor_sync(FULL, alpha, 4);
         if (state == Q_LINE && both) {

@@ -52,3 +52,65 @@ def test_solves_match_oracle(n, blk):
     ce, co = e.counters(), o.counters()
     assert ce["pairs_solved"] == co["pairs_solved"] and ce["pairs_solved"] > 0 or n < 8
     assert abs(ce["iters"] - co["iters"]) <= max(2, 0.01 * co["iters"])
+
+
+SUMS = r"""
+#include <cuda_runtime.h>
+#include "gb2_mlp.cuh"
+#include "gb2_sq_solve.cuh"
+__global__ void k(const double *a, const double *b, double *s4, double *s8)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    s4[i] = gb2::sq::sum4(0xffffffffu, a[i] * 0.5, b[i]);   // a product the compiler could contract further
+    s8[i] = gb2::sq::sum8(0xffffffffu, a[i], b[i]);
+}
+extern "C" int run(const double *a, const double *b, int n, double *s4, double *s8)
+{
+    double *d;
+    if (cudaMalloc(&d, n * 32)) return 1;
+    cudaMemcpy(d, a, n * 8, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + n, b, n * 8, cudaMemcpyHostToDevice);
+    k<<<n / 128, 128>>>(d, d + n, d + 2 * n, d + 3 * n);
+    cudaMemcpy(s4, d + 2 * n, n * 8, cudaMemcpyDeviceToHost);
+    const int rc = cudaMemcpy(s8, d + 3 * n, n * 8, cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(d);
+    return rc;
+}
+"""
+
+
+def _contracted(a, b):
+    """What a fused multiply-add in each lane's first butterfly step would give
+    (own product unrounded, partner's rounded), by exact rational arithmetic."""
+    from fractions import Fraction
+    p = a * b
+    own = [float(Fraction(x) * Fraction(y) + Fraction(q)) for x, y, q in zip(a, b, p.reshape(-1, 2)[:, ::-1].ravel())]
+    return np.array(own)
+
+
+def test_group_sums_are_the_same_in_every_lane(tmp_path):
+    """The solver's control flow rests on it.  Built with the flags of the
+    superquadric unit, contraction on: the contracted form differs between the
+    two lanes of a pair for these operands (checked here on the host)."""
+    import ctypes
+    import subprocess
+    csrc = os.path.join(HERE, "..", "liggghts-public_b200", "csrc")
+    src, so = tmp_path / "t.cu", tmp_path / "t.so"
+    src.write_text(SUMS)
+    subprocess.run(["nvcc", "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", csrc, "-shared",
+                    "-Xcompiler", "-fPIC", "-o", str(so), str(src)], check=True)
+    lib, n = ctypes.CDLL(str(so)), 128 * 64
+    rng = np.random.default_rng(11)
+    a, b = (rng.uniform(-1, 1, n) * 10.0 ** rng.uniform(-6, 6, n) for _ in range(2))
+    s4, s8 = np.empty(n), np.empty(n)
+    P = lambda v: v.ctypes.data_as(ctypes.POINTER(ctypes.c_double))  # noqa: E731
+    assert lib.run(P(a), P(b), n, P(s4), P(s8)) == 0
+    def butterfly(p, lanes):
+        p = p.reshape(-1, lanes)
+        while p.shape[1] > 1:
+            p = p[:, 0::2] + p[:, 1::2]
+        return np.repeat(p[:, 0], lanes)
+    assert np.array_equal(s4, butterfly((a * 0.5) * b, 4))
+    assert np.array_equal(s8, butterfly(a * b, 8))
+    c = _contracted(a[:512], b[:512]).reshape(-1, 2)
+    assert (c[:, 0] != c[:, 1]).any()
