@@ -50,7 +50,7 @@ def test_solves_match_oracle(n, blk):
         for k in ("f", "torque"):
             assert np.abs(f[k] - g[k]).max() <= 1e-5 * max(np.abs(g[k]).max(), 1e-30)
     ce, co = e.counters(), o.counters()
-    assert ce["pairs_solved"] == co["pairs_solved"] and ce["pairs_solved"] > 0 or n < 8
+    assert ce["pairs_solved"] == co["pairs_solved"] and (ce["pairs_solved"] > 0 or n < 8)
     assert abs(ce["iters"] - co["iters"]) <= max(2, 0.01 * co["iters"])
 
 
