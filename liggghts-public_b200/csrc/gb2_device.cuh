@@ -9,7 +9,6 @@
 #include "gb2_internal.h"
 
 namespace gb2 {
-__device__ __forceinline__ dbl4 ld4(const dbl4 *p) { return *p; }
 
 __device__ __forceinline__ flt8 make_kin(const dbl4 &v, const dbl4 &w)
 {
@@ -230,24 +229,37 @@ __device__ __forceinline__ bool coplanar_node_neighs(const MeshDev &M, int a, in
 // bit mask; the compute phase then evaluates only touching entries, in list
 // order, so the per-atom sums keep the reference's order.
 
-// One 32-byte record through the read-only path as a single 256-bit load
-// (sm_100 vector width): a scattered warp-wide gather then needs one L1
-// wavefront per lane's line instead of two.  Records are 32-byte aligned.
-__device__ __forceinline__ dbl4 ldg4(const dbl4 *p)
+// One 32-byte record as a single 256-bit load (sm_100 vector width): a
+// scattered warp-wide gather then needs one L1 wavefront per lane's line
+// instead of two.  Records are 32-byte aligned.  Ordinary loads, not read-only
+// ones (ld.global.nc): the pair step and the tail kernel may be launched while
+// the kernel that writes these records still runs, so the records are constant
+// after their griddepcontrol.wait, not for the kernel's whole life.  volatile
+// keeps the loads behind that wait.
+__device__ __forceinline__ dbl4 ldrec(const dbl4 *p)
 {
     dbl4 r;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
     return r;
 }
 
-// One split-precision kinematics record (eight FP32 values) as one 256-bit
-// read-only load.
-__device__ __forceinline__ flt8 ldg8f(const flt8 *p)
+// The same from L2, for what a kernel reads before its wait: the records of
+// the previous step are complete by then (the tail kernel is launched once
+// the pair step has waited for them), but L1 may hold an older copy.
+__device__ __forceinline__ dbl4 ldrec_l2(const dbl4 *p)
+{
+    dbl4 r;
+    asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
+
+// One split-precision kinematics record (eight FP32 values) as one 256-bit load.
+__device__ __forceinline__ flt8 ldkin(const flt8 *p)
 {
     flt8 r;
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(r.vx), "=f"(r.vy), "=f"(r.vz), "=f"(r.m), "=f"(r.wx), "=f"(r.wy), "=f"(r.wz), "=f"(r.pad)
-        : "l"(p));
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.vx), "=f"(r.vy), "=f"(r.vz), "=f"(r.m), "=f"(r.wx), "=f"(r.wy), "=f"(r.wz), "=f"(r.pad)
+                 : "l"(p));
     return r;
 }
 
@@ -317,10 +329,10 @@ __device__ __forceinline__ void screen_both(const Dev &D, int k, int nr, int nn,
     int b0 = (0 < nn) ? ld_stream(&D.nbr[k]) : k;
     int b1 = (1 < nn) ? ld_stream(&D.nbr[cap + k]) : k;
     for (int t = 0; t < n; t += 2) {
-        const dbl4 qa0 = ldg4(&D.pos[a0]);
-        const dbl4 qa1 = ldg4(&D.pos[a1]);
-        const dbl4 qb0 = ldg4(&D.pos[b0]);
-        const dbl4 qb1 = ldg4(&D.pos[b1]);
+        const dbl4 qa0 = ldrec(&D.pos[a0]);
+        const dbl4 qa1 = ldrec(&D.pos[a1]);
+        const dbl4 qb0 = ldrec(&D.pos[b0]);
+        const dbl4 qb1 = ldrec(&D.pos[b1]);
         const int u = t + 2;
         a0 = (u < nr) ? ld_stream(&D.rev[u * cap + k]) : k;
         a1 = (u + 1 < nr) ? ld_stream(&D.rev[(u + 1) * cap + k]) : k;
@@ -385,8 +397,8 @@ __device__ __forceinline__ bool screen_list(const Dev &D, int k, int nr, int nn,
             const int b1 = t1 < nn ? ld_stream(&D.nbr[t1 * cap + k]) : 0;
             const int s0 = t0 < nr ? (int)D.revs[t0 * cap + k] : 0;
             const int s1 = t1 < nr ? (int)D.revs[t1 * cap + k] : 0;
-            const dbl4 qa0 = ldg4(&D.pos[a0]), qa1 = ldg4(&D.pos[a1]);
-            const dbl4 qb0 = ldg4(&D.pos[b0]), qb1 = ldg4(&D.pos[b1]);
+            const dbl4 qa0 = ldrec(&D.pos[a0]), qa1 = ldrec(&D.pos[a1]);
+            const dbl4 qb0 = ldrec(&D.pos[b0]), qb1 = ldrec(&D.pos[b1]);
             const bool ta0 = t0 < nr && touching(pk, qa0), ta1 = t1 < nr && touching(pk, qa1);
             const bool tb0 = t0 < nn && touching(pk, qb0), tb1 = t1 < nn && touching(pk, qb1);
             if (ta0) mrev |= 1ull << t0;
@@ -416,10 +428,10 @@ __device__ __forceinline__ bool screen_list(const Dev &D, int k, int nr, int nn,
         int b0 = (0 < nn) ? ld_stream(&D.nbr[k]) : 0;
         int b1 = (1 < nn) ? ld_stream(&D.nbr[cap + k]) : 0;
         for (int t = 0; t < nw; t += 2) {
-            const dbl4 qa0 = ldg4(&D.pos[a0]);
-            const dbl4 qa1 = ldg4(&D.pos[a1]);
-            const dbl4 qb0 = ldg4(&D.pos[b0]);
-            const dbl4 qb1 = ldg4(&D.pos[b1]);
+            const dbl4 qa0 = ldrec(&D.pos[a0]);
+            const dbl4 qa1 = ldrec(&D.pos[a1]);
+            const dbl4 qb0 = ldrec(&D.pos[b0]);
+            const dbl4 qb1 = ldrec(&D.pos[b1]);
             const int ca0 = a0, ca1 = a1, cs0 = s0, cs1 = s1, cb0 = b0, cb1 = b1;
             const int u = t + 2;
             a0 = (u < nr) ? ld_stream(&D.rev[u * cap + k]) : 0;
@@ -452,8 +464,8 @@ __device__ __forceinline__ bool screen_list(const Dev &D, int k, int nr, int nn,
             int ca[U], cb[U], cs[U];
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                qa[u] = ldg4(&D.pos[a[u]]);
-                qb[u] = ldg4(&D.pos[b[u]]);
+                qa[u] = ldrec(&D.pos[a[u]]);
+                qb[u] = ldrec(&D.pos[b[u]]);
                 ca[u] = a[u];
                 cb[u] = b[u];
                 cs[u] = sl[u];

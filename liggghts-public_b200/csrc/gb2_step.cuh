@@ -36,15 +36,17 @@ constexpr int kTailAtoms = GB2_TAIL_ATOMS;
 // list otherwise).  A j-side entry is evaluated from kk's side with the
 // shear negated; an own entry updates kk's shear slot in the write buffer
 // and sets the contact flag.  res receives the pair's force and torque on kk.
-template <bool ROLLING, bool SPLIT, bool ONE, typename Real>
+// EARLY: called before the kernel's wait, so the records come from L2.
+template <bool ROLLING, bool SPLIT, bool ONE, bool EARLY = false, typename Real>
 __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s, bool own, bool upd, Real *res)
 {
     const int cap = D.cap;
     const int e = s * cap + kk;
     const double sgn = own ? 1.0 : -1.0;
     const int hrow = own ? kk : other;
-    const dbl4 pkk = ldg4(&D.pos[kk]);
-    const dbl4 po = ldg4(&D.pos[other]);
+    const auto ld = [](const dbl4 *p) { return EARLY ? ldrec_l2(p) : ldrec(p); };
+    const dbl4 pkk = ld(&D.pos[kk]);
+    const dbl4 po = ld(&D.pos[other]);
     const double delx = pkk.x - po.x;
     const double dely = pkk.y - po.y;
     const double delz = pkk.z - po.z;
@@ -52,13 +54,13 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
     // material lookup in the reference's (owner, neighbour) order
     const MatPair &M = ONE ? D.mat1 : (own ? mat(D, D.type[kk], D.type[other]) : mat(D, D.type[other], D.type[kk]));
     if constexpr (SPLIT) {
-        const flt8 a = ldg8f(&D.kin[kk]), b = ldg8f(&D.kin[other]);
+        const flt8 a = ldkin(&D.kin[kk]), b = ldkin(&D.kin[other]);
         const double r = sqrt(rsq);
         const double deltan = (pkk.w + po.w) - r;   // FP64 overlap
         const float va[3] = {a.vx, a.vy, a.vz}, wa[3] = {a.wx, a.wy, a.wz};
         const float vb[3] = {b.vx, b.vy, b.vz}, wb[3] = {b.wx, b.wy, b.wz};
         const float fs = (float)sgn;
-        const dbl4 h = ldg4(&D.hist[s * cap + hrow]);
+        const dbl4 h = ld(&D.hist[s * cap + hrow]);
         float sh[3] = {fs * (float)h.x, fs * (float)h.y, fs * (float)h.z};
         ContactOutF o;
         pair_contact_f32(M, (float)delx, (float)dely, (float)delz, (float)r, (float)deltan, (float)pkk.w,
@@ -69,26 +71,30 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
             res[3 + c] = o.T[c];
         }
     } else {
-        const dbl4 vk4 = ldg4(&D.vel[kk]), wk4 = ldg4(&D.omg[kk]);
-        const dbl4 vo4 = ldg4(&D.vel[other]), wo4 = ldg4(&D.omg[other]);
+        const dbl4 vk4 = ld(&D.vel[kk]), wk4 = ld(&D.omg[kk]);
+        const dbl4 vo4 = ld(&D.vel[other]), wo4 = ld(&D.omg[other]);
         const double vk[3] = {vk4.x, vk4.y, vk4.z}, wk[3] = {wk4.x, wk4.y, wk4.z};
         const double vo[3] = {vo4.x, vo4.y, vo4.z}, wo[3] = {wo4.x, wo4.y, wo4.z};
-        const dbl4 h = ldg4(&D.hist[s * cap + hrow]);
+        const dbl4 h = ld(&D.hist[s * cap + hrow]);
         double sh[3] = {sgn * h.x, sgn * h.y, sgn * h.z};   // exact: multiplying by +-1 only flips the sign
         ContactOut o;
         if (!pair_contact_fast(M, delx, dely, delz, rsq, pkk.w, po.w, vk, vo, wk, wo, vk4.w, vo4.w, sh, upd, D.dt,
                                ROLLING, D.tdamp != 0, o)) {
             // an operand outside the fast arithmetic's range: read again, so that
             // this rare path keeps nothing alive through the other
-            const dbl4 p1 = D.pos[kk], p2 = D.pos[other], v1 = D.vel[kk], v2 = D.vel[other], w1 = D.omg[kk],
-                       w2 = D.omg[other], h1 = D.hist[s * cap + hrow];
+            const auto again = [](const dbl4 *p) { return EARLY ? ldrec_l2(p) : *p; };
+            const dbl4 p1 = again(&D.pos[kk]), p2 = again(&D.pos[other]), v1 = again(&D.vel[kk]),
+                       v2 = again(&D.vel[other]), w1 = again(&D.omg[kk]), w2 = again(&D.omg[other]),
+                       h1 = again(&D.hist[s * cap + hrow]);
+            const auto type_again = [&D](int a) { return *(const volatile int *)&D.type[a]; };
             const double dx = p1.x - p2.x, dy = p1.y - p2.y, dz = p1.z - p2.z;
             const double va[3] = {v1.x, v1.y, v1.z}, vb[3] = {v2.x, v2.y, v2.z};
             const double wa[3] = {w1.x, w1.y, w1.z}, wb[3] = {w2.x, w2.y, w2.z};
             sh[0] = sgn * h1.x;
             sh[1] = sgn * h1.y;
             sh[2] = sgn * h1.z;
-            pair_contact<false>(M, dx, dy, dz, dx * dx + dy * dy + dz * dz, p1.w, p2.w, va, vb, wa, wb, v1.w, v2.w, sh,
+            const MatPair &M1 = ONE ? D.mat1 : mat(D, type_again(own ? kk : other), type_again(own ? other : kk));
+            pair_contact<false>(M1, dx, dy, dz, dx * dx + dy * dy + dz * dz, p1.w, p2.w, va, vb, wa, wb, v1.w, v2.w, sh,
                                 upd, D.dt, ROLLING, D.tdamp != 0, o);
         }
         if (own && upd) D.hist_out[e] = dbl4{(double)sh[0], (double)sh[1], (double)sh[2], 0.0};
@@ -103,10 +109,15 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
 // whole warp: the entries of a side are screened 128 at a time, the touching
 // ones listed in order (list: kLongList ints of the warp's shared memory),
 // evaluated one per lane, and added in list order -- the reference's order --
-// by every lane.  Out of line, so the tail kernel's registers are its own.  What bounds it is the chain of dependent gathers, so the
+// by every lane.  What bounds it is the chain of dependent gathers, so the
 // entries of four chunks are in flight together; one lane taking the entries
 // one by one (a 3 mm sphere in a bed of 0.3 mm spheres has hundreds) set the
-// whole step's time.  FP64 in both precisions.
+// whole step's time.  Out of line, as inlined it would take part in the tail
+// kernel's register allocation; the call has its price too (the tail kernel
+// keeps more of its state in local memory around it than it does without, and
+// took 41.6 us a launch instead of 39.7 on the packed 1M hopper, which has no
+// such atom).  FP64 in both precisions, records from L2 (called before the
+// wait).
 constexpr int kLongList = kTailAtoms * 64;
 
 template <bool ROLLING>
@@ -114,7 +125,7 @@ __device__ __noinline__ void long_atom(const Dev &D, int k, int nr, int nn, bool
 {
     const unsigned FULL = 0xffffffffu;
     const int cap = D.cap, lane = threadIdx.x & 31;
-    const dbl4 pk = ldg4(&D.pos[k]);
+    const dbl4 pk = ldrec_l2(&D.pos[k]);
     for (int c = 0; c < 3; c++) acc.F[c] = acc.T[c] = 0.0;
     for (int side = 0; side < 2; side++) {
         const int tot = side ? nn : nr;
@@ -129,12 +140,12 @@ __device__ __noinline__ void long_atom(const Dev &D, int k, int nr, int nn, bool
                 j[u] = e < tot ? ld_stream(&idx[e * cap + k]) : k;
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) q[u] = ldg4(&D.pos[j[u]]);
+            for (int u = 0; u < 4; u++) q[u] = ldrec_l2(&D.pos[j[u]]);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const int e = base + 32 * u + lane;
                 const bool t = e < tot && touching(pk, q[u]);
-                if (side && upd && e < tot && !t) D.hist_out[e * cap + k] = ldg4(&D.hist[e * cap + k]);
+                if (side && upd && e < tot && !t) D.hist_out[e * cap + k] = ldrec_l2(&D.hist[e * cap + k]);
                 const unsigned m = __ballot_sync(FULL, t);
                 if (t) list[n + __popc(m & ((1u << lane) - 1u))] = e;
                 n += __popc(m);
@@ -146,8 +157,9 @@ __device__ __noinline__ void long_atom(const Dev &D, int k, int nr, int nn, bool
                     if (b + lane < n) {
                         const int e = list[b + lane];
                         const int s = side ? e : (int)D.revs[e * cap + k];
-                        if (side) D.flag[e * cap + k] |= 5;   // CONTACT_NORMAL_MODEL | CONTACT_TANGENTIAL_MODEL
-                        eval_item<ROLLING, false, false>(D, k, __ldg(&idx[e * cap + k]), s, side == 1, upd, res);
+                        if (side)   // CONTACT_NORMAL_MODEL | CONTACT_TANGENTIAL_MODEL
+                            D.flag[e * cap + k] = __ldcg(&D.flag[e * cap + k]) | 5;
+                        eval_item<ROLLING, false, false, true>(D, k, __ldg(&idx[e * cap + k]), s, side == 1, upd, res);
                     }
                     const int cnt = min(32, n - b);
                     for (int t = 0; t < cnt; t++)
@@ -336,7 +348,7 @@ __device__ __forceinline__ void atom_hist_tail(const Dev &D, int k, unsigned lon
     while (stopped) {
         const int s = __ffsll((long long)stopped) - 1;
         stopped &= stopped - 1ull;
-        D.hist_out[s * cap + k] = ldg4(&D.hist[s * cap + k]);
+        D.hist_out[s * cap + k] = ldrec(&D.hist[s * cap + k]);
     }
     D.prevmask[k] = mown;
 }
@@ -583,9 +595,9 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ De
         pi = vi4 = wi4 = hold = dbl4{0.0, 0.0, 0.0, 0.0};
         if (own) {
             i = D.tail[base + lane];
-            pi = D.pos[i];
-            vi4 = D.vel[i];
-            wi4 = D.omg[i];
+            pi = ldrec_l2(&D.pos[i]);
+            vi4 = ldrec_l2(&D.vel[i]);
+            wi4 = ldrec_l2(&D.omg[i]);
             if (fuse_next) hold = D.xhold[i];
             ti = D.type[i];
             nr = D.rnum[i];
