@@ -1231,12 +1231,13 @@ int do_rebuild(gb2_ctx *c, bool pre_exchange, bool sort_now, bool insert, bool g
             k_tail_list<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D3);
             CKL();
         }
-        if (checked) break;
         // the last look at the device: the meshes' slots, and the count of
-        // short item lists for adapt_item_cap
+        // short item lists for adapt_item_cap.  Every build ends behind this
+        // synchronisation: the pair step reads the list lengths and tflag
+        // before its wait for the kernel in front of it, which may be one of these.
         CK(cudaMemcpyAsync(&c->h_pinned[6], c->dneed.p + 4, sizeof(int), cudaMemcpyDeviceToHost, c->st));
         if (read_status(c, &st)) return GB2_ERR_CUDA;
-        if (!(st & ST_MESHSLOT_OVERFLOW)) {
+        if (checked || !(st & ST_MESHSLOT_OVERFLOW)) {
             if (st & ST_MESH_INTERNAL) return set_err(c, GB2_ERR_STATE, "mesh contact history inconsistent");
             break;
         }

@@ -421,7 +421,8 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     unsigned long long mrev = 0ull, mown = 0ull;
     bool serial = false, tail = false;
     // what changes only at a build is read while the previous step's tail
-    // kernel still runs (this grid is its programmatic dependent)
+    // kernel still runs (this grid is its programmatic dependent; the host
+    // synchronises behind a build before it launches the next pair step)
     if (valid) {
         nr = D.rnum[k];
         nn = D.nnum[k];
