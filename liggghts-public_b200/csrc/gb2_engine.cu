@@ -1090,10 +1090,12 @@ int do_build(gb2_ctx *c)
     return 0;
 }
 
-//
 // checked false: nothing is read back; the caller looks at the status word
 // later and, on ST_MESHSLOT_OVERFLOW, takes the new slots back
 // (undo_pre_force) and calls again with checked true, which grows the slots.
+// The re-paging empties slots of the old arrays, so it must not see a cut
+// candidate list: every mesh's candidates are listed before the first
+// re-paging, which does nothing once a list did not fit (k_mesh_repage).
 int do_pre_force(gb2_ctx *c, bool checked)
 {
     // FixWallGran::pre_force, FixNeighlistMesh::pre_force,
@@ -1131,7 +1133,6 @@ int do_pre_force(gb2_ctx *c, bool checked)
         if (H.kind == FIX_WALL_MESH) {
             MeshFix &M = *H.mesh;
             // candidates into fresh buffers (old slots are still needed)
-            const int old_maxt = M.maxt;
             CK(M.tcnt2.alloc(c->cap));
             M.tcnt.swap(M.tcnt2);   // the old counts are not needed by the re-paging
             for (int attempt = 0; attempt < 8; attempt++) {
@@ -1148,6 +1149,12 @@ int do_pre_force(gb2_ctx *c, bool checked)
                 M.maxt = grown_capacity(c, 3, M.maxt, 64);
                 M.tlist.release();
             }
+        }
+    }
+    for (int k = 0; k < c->nfix; k++) {
+        HostFix &H = c->fix[k];
+        if (H.kind == FIX_WALL_MESH) {
+            MeshFix &M = *H.mesh;
             // re-page history into buffers sized for the new capacity
             CK(M.snp2.alloc(c->cap));
             CK(M.spartner2.alloc((size_t)M.maxt * c->cap));
@@ -1158,7 +1165,7 @@ int do_pre_force(gb2_ctx *c, bool checked)
             if (checked && clear_status(c)) return GB2_ERR_CUDA;
             Dev D = make_dev(c);
             // old slots now live in *2 buffers
-            k_mesh_repage<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D, k, M.snp2.p, M.spartner2.p, M.shist2.p, old_maxt);
+            k_mesh_repage<<<nblk(c->nlocal), kBlock, 0, c->st>>>(D, k, M.snp2.p, M.spartner2.p, M.shist2.p);
             CKL();
             if (!checked) continue;
             int st;
@@ -1169,7 +1176,8 @@ int do_pre_force(gb2_ctx *c, bool checked)
     return 0;
 }
 
-// the meshes' contact slots as they were before do_pre_force
+// the meshes' contact slots as they were before an unchecked do_pre_force
+// whose candidates did not fit
 void undo_pre_force(gb2_ctx *c)
 {
     for (int k = 0; k < c->nfix; k++) {

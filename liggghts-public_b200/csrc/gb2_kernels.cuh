@@ -604,8 +604,11 @@ __global__ void k_mesh_sort_contacts(Dev D, int ifix)
 // FixContactHistoryMesh::pre_force with cleanUpContactJumps
 // (src/fix_contact_history_mesh.cpp:315-373, :466-508).  Reads the old slot
 // arrays (oldM) and writes re-paged slots sized to the new candidate count.
-__global__ void k_mesh_repage(Dev D, int ifix, int *old_snp, int *old_spartner, double *old_shist, int old_maxt)
+__global__ void k_mesh_repage(Dev D, int ifix, int *old_snp, int *old_spartner, double *old_shist)
 {
+    // a candidate list of some mesh was cut at its capacity (the kernels before
+    // this one on the stream): the old slots are needed again, as they are
+    if (*(volatile int *)D.status & ST_MESHSLOT_OVERFLOW) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= D.nlocal) return;
     const MeshDev &M = D.fix[ifix].mesh;
@@ -639,7 +642,6 @@ __global__ void k_mesh_repage(Dev D, int ifix, int *old_snp, int *old_spartner, 
         } else
             ip++;
     }
-    (void)old_maxt;
     if (np > nn) atomicOr(D.status, ST_MESH_INTERNAL);
     for (int k = 0; k < nn; k++) {
         int t = -1;
