@@ -2380,6 +2380,12 @@ int gb2_run(gb2_ctx *c, int nsteps)
             int rc = one_step(c, s == nsteps - 1, 1);
             if (rc) return rc;
             s++;
+        } else if (stop) {
+            // asked on the run's last step: by a mesh (the atoms' test is part of
+            // the next step's integration, which the last step does not start),
+            // and the request stands for the next run
+            for (int k = 0; k < c->nfix; k++)
+                if (c->fix[k].mesh && c->fix[k].mesh->moving) c->fix[k].mesh->next_reneighbor = c->ntimestep + 1;
         }
     }
     int st;
