@@ -327,6 +327,7 @@ __device__ __forceinline__ void atom_store_integrate(const Dev &D, int i, const 
 // fix insert/stream holds, set in place once the step's kernels are done.
 static __global__ void k_stream_positions(Dev D)
 {
+    if (step_cancelled(D)) return;   // D.pos is then an earlier step's
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= D.nlocal) return;
     dbl4 x = D.pos[i], v, w;

@@ -59,3 +59,24 @@ def test_mesh_asks_on_the_last_step(monkeypatch):
         qn, rn = q.mesh_nodes(1), r.mesh_nodes(1)
         assert np.array_equal(qn[0], rn[0]) and np.array_equal(qn[1], rn[1])
     assert contacts > 0
+
+
+@pytest.mark.parametrize("after", [1, 2, 3, 4, 5])
+def test_stream_run_ends_after_a_request(monkeypatch, after):
+    """Particles that fix insert/stream holds, pushed into free ones below its face; every run ends `after` steps
+    after a step that asked for a rebuild."""
+    sc = S.stream_pour(n_bed=200)
+    x = sc["atoms"]["x"]
+    x[:60, 2] = 0.0385 + 0.5e-3 * (np.arange(60) % 3)
+    builds = [b for b in _build_steps(_engine(sc, monkeypatch, 0), 320)]
+    asked = [b - 1 for b in builds if (b - 1) % 200 > 5]
+    q, r = _engine(sc, monkeypatch, None), _engine(sc, monkeypatch, 0)
+    held = 0
+    for n in _segments([a + after for a in asked if a > 8]):
+        q.run(n)
+        r.run(n)
+        assert q.stats()["nbuilds"] == r.stats()["nbuilds"]
+        assert_atoms_equal(q, r)
+        assert_pairs_equal(q, r)
+        held += 1
+    assert held > 5 and len(q.atoms()["x"]) > 200
