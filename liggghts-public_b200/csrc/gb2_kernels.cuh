@@ -207,7 +207,8 @@ __global__ void k_pbc(Dev D, double lo0, double lo1, double lo2, double hi0, dou
     D.pos[i] = p;
 }
 
-// Atom::sort keys (src/atom.cpp:1343-1354)
+// Atom::sort keys (src/atom.cpp:1343-1354), with the arrivals per bin counted
+// for a counting sort (counts) or the indices for a sort of pairs (null)
 __global__ void k_sort_keys(Dev D, double lo0, double lo1, double lo2, double inv0, double inv1, double inv2, int nb0,
                             int nb1, int nb2, unsigned *keys, int *vals, int *counts)
 {
@@ -223,16 +224,18 @@ __global__ void k_sort_keys(Dev D, double lo0, double lo1, double lo2, double in
     ix = min(ix, nb0 - 1);
     iy = min(iy, nb1 - 1);
     iz = min(iz, nb2 - 1);
-    const int b = iz * nb1 * nb0 + iy * nb0 + ix;
-    keys[i] = static_cast<unsigned>(b);
-    vals[i] = atomicAdd(&counts[b], 1);   // its place among the bin's arrivals
+    const unsigned b = ((unsigned)iz * nb1 + iy) * (unsigned)nb0 + ix;
+    keys[i] = b;
+    vals[i] = counts ? atomicAdd(&counts[b], 1) : i;   // its place among the bin's arrivals, or itself
 }
 
 // The atoms in bin order, ascending within a bin: a counting sort whose
 // arrival order (k_bin_scatter; start is the scan of the counts) is replaced
-// by the rank of each atom among its bin's (k_bin_rank).  Bins hold an atom or
-// two, so this reads and writes each atom a few times where a radix sort takes
-// three or four passes of ~10 us even for a thousand atoms.
+// by the rank of each atom among its bin's (k_bin_rank), which reads the whole
+// bin: for bins no wider than the list cutoff, whose atoms the list build reads
+// again anyway.  They mostly hold an atom or two, so this reads and writes each
+// atom a few times where a radix sort takes three or four passes of ~10 us even
+// for a thousand atoms.
 __global__ void k_bin_scatter(int n, const unsigned *__restrict__ keys, const int *__restrict__ arrival,
                               const int *__restrict__ start, int *__restrict__ out)
 {
