@@ -275,7 +275,7 @@ __device__ __forceinline__ bool pair_contact_fast(const MatPair &M, double delx,
         Ft2 *= ratio;
         Ft3 *= ratio;
         if (update_history) {
-            ok = ok & fast_range(fabs(Ft1)) & fast_range(fabs(Ft2)) & fast_range(fabs(Ft3)) & fast_divisor(kt);
+            ok = ok & fast_range0(fabs(Ft1)) & fast_range0(fabs(Ft2)) & fast_range0(fabs(Ft3)) & fast_divisor(kt);
             const double ktinv = fast_rcp(kt);
             shear[0] = fast_quot(-Ft1, kt, ktinv);
             shear[1] = fast_quot(-Ft2, kt, ktinv);
