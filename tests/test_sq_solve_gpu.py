@@ -114,3 +114,38 @@ def test_group_sums_are_the_same_in_every_lane(tmp_path):
     assert np.array_equal(s8, butterfly(a * b, 8))
     c = _contracted(a[:512], b[:512]).reshape(-1, 2)
     assert (c[:, 0] != c[:, 1]).any()
+
+
+def _aligned_boxes(n, blk, seed=5):
+    """Particles of one orientation, faces nearly parallel and nearly flat, in slight overlap."""
+    sc = S.sq_packing(n=n, seed=seed)
+    a, rng = sc["atoms"], np.random.default_rng(seed + 1)
+    a["blockiness"] = np.full(n, blk)
+    a["quat"][:] = S.random_quaternions(rng, 1)[0]
+    w, x, y, z = a["quat"][0]
+    R = np.array([[w * w + x * x - y * y - z * z, 2 * (x * y - w * z), 2 * (x * z + w * y)],
+                  [2 * (x * y + w * z), w * w - x * x + y * y - z * z, 2 * (y * z - w * x)],
+                  [2 * (x * z - w * y), 2 * (y * z + w * x), w * w - x * x - y * y + z * z]])
+    a["shape"][:] = 1.5e-3 * rng.uniform(0.8, 1.2, (n, 3))
+    vol = S.sq_volume(a["shape"], a["blockiness"])
+    a.update(rmass=vol * 2500.0, inertia=S.sq_inertia(a["shape"], a["blockiness"], 2500.0), volume=vol)
+    m, i = int(np.ceil(n ** (1 / 3))), np.arange(n)
+    g = np.stack([i % m, (i // m) % m, i // (m * m)], axis=1).astype(float)
+    a["x"] = np.ascontiguousarray((g * 3e-3 * 0.97 + rng.uniform(-4e-4, 4e-4, (n, 3))) @ R.T)
+    return sc
+
+
+@pytest.mark.parametrize("blk,tol", [(4.0, 0.002), (8.0, 0.04), (12.0, 0.08)])
+def test_flat_faces_take_the_oracles_iterations(blk, tol):
+    """Where the Hessians are nearly singular the Newton steps have to be those of pivoted elimination, as in the
+    oracle: the first contacts take its iterations (steps from cofactors alone took 8 % fewer at blockiness 8 and
+    27 % fewer at 12, in the oracle's own arithmetic, and left more solves unconverged)."""
+    import granb200
+    sc = _aligned_boxes(64, blk)
+    e, o = granb200.SqEngine(sc), oracle.SqOracle(sc)
+    e.setup()
+    o.setup()
+    ce, co = e.counters(), o.counters()
+    print(blk, ce, co)
+    assert ce["pairs_solved"] == co["pairs_solved"] > 100 and ce["solves"] == co["solves"]
+    assert abs(ce["iters"] - co["iters"]) <= tol * co["iters"]
