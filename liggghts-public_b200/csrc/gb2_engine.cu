@@ -163,6 +163,7 @@ struct gb2_ctx {
     DBuf<flt8> kin, kin2;         // split precision: FP32 kinematics records (double-buffered like vel)
     DBuf<uint8_t> revs, tflag;
     int nsm = 148;                // SMs of the device
+    int pair_lanes = 0;           // lanes per atom of the FP64 pair step (0: by the number of atoms)
     int tail_per_sm = 8;          // blocks of the tail kernel per SM (kTailAtoms atoms per warp)
     int item_cap = 160;           // listed-round capacity per warp and side (grown on demand up to kItemCap)
     bool item_cap_fixed = false;  // GB2_ITEM_CAP sets it and stops the growth (0: masks only)
@@ -1316,7 +1317,8 @@ void launch_pair(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int f
     // hopper 32.1 -> 31.0).  At 40,000 spheres both take the same, at 300,000
     // two lanes are slower (83 -> 102).  Four lanes gain nothing on two.
     // Split precision keeps one lane: its results would change in their last bits.
-    const int lanes = !c->split && c->nlocal <= 200 * c->nsm ? 2 : 1;
+    // GB2_PAIR_LANES fixes the number (the results are the same).
+    const int lanes = c->pair_lanes ? c->pair_lanes : (!c->split && c->nlocal <= 200 * c->nsm ? 2 : 1);
     if (c->split)
         launch_pair_split(D, c->st, shearupdate, integrate, fuse_next, store_f, pair_list_smem(c));
     else
@@ -1460,6 +1462,7 @@ int gb2_create(const gb2_params *p, gb2_ctx **out)
     c->P = *p;
     c->split = p->precision == GB2_PREC_SPLIT;
     if (c->P.neigh_every <= 0) c->P.neigh_every = 1;
+    if (const char *pl = std::getenv("GB2_PAIR_LANES")) c->pair_lanes = std::min(std::max(std::atoi(pl), 0), 2);
     if (const char *tb = std::getenv("GB2_TAIL_BLOCKS")) c->tail_per_sm = std::max(1, std::atoi(tb));
     if (const char *ic = std::getenv("GB2_ITEM_CAP")) {
         c->item_cap = std::min(std::max(std::atoi(ic), 0), kItemCap);
