@@ -163,6 +163,7 @@ struct gb2_ctx {
     DBuf<flt8> kin, kin2;         // split precision: FP32 kinematics records (double-buffered like vel)
     DBuf<uint8_t> revs, tflag;
     int nsm = 148;                // SMs of the device
+    bool long_lists = true;       // some atom has more than 64 entries on a side (since the last build)
     int pair_lanes = 0;           // lanes per atom of the FP64 pair step (0: by the number of atoms)
     int tail_per_sm = 8;          // blocks of the tail kernel per SM (kTailAtoms atoms per warp)
     int item_cap = 160;           // listed-round capacity per warp and side (grown on demand up to kItemCap)
@@ -1269,6 +1270,7 @@ int do_rebuild(gb2_ctx *c, bool pre_exchange, bool sort_now, bool insert, bool g
         if (read_status(c, &st)) return GB2_ERR_CUDA;
         if (checked || !(st & ST_MESHSLOT_OVERFLOW)) {
             if (st & ST_MESH_INTERNAL) return set_err(c, GB2_ERR_STATE, "mesh contact history inconsistent");
+            c->long_lists = (st & ST_LONG_LISTS) != 0;
             break;
         }
         undo_pre_force(c);
@@ -1329,11 +1331,8 @@ void launch_pair(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int f
 void launch_tail(gb2_ctx *c, const Dev &D, int shearupdate, int integrate, int fuse_next, int store_f)
 {
     const int tblocks = c->tail_per_sm * c->nsm;
-    if (c->split) launch_tail_split(D, tblocks, c->st, shearupdate, integrate, fuse_next, store_f);
-    else if (c->P.rolling_cdt)
-        launch_pair_tail<true, false>(D, tblocks, c->st, shearupdate, integrate, fuse_next, store_f);
-    else
-        launch_pair_tail<false, false>(D, tblocks, c->st, shearupdate, integrate, fuse_next, store_f);
+    if (c->split) launch_tail_split(D, c->long_lists, tblocks, c->st, shearupdate, integrate, fuse_next, store_f);
+    else launch_pair_tail<false>(D, c->long_lists, tblocks, c->st, shearupdate, integrate, fuse_next, store_f);
 }
 
 int do_force(gb2_ctx *c, int shearupdate, int integrate, int fuse_next, int store_f)

@@ -59,6 +59,7 @@ enum : int {
     ST_REV_OVERFLOW = 1 << 4,
     ST_MESH_INTERNAL = 1 << 5,
     ST_MESH_OUTSIDE_GRID = 1 << 6,
+    ST_LONG_LISTS = 1 << 7,   // some atom has more than 64 entries on a side (set at a build, no error)
 };
 
 enum FixKind : int { FIX_NONE = 0, FIX_GRAVITY = 1, FIX_WALL_PLANE = 2, FIX_WALL_MESH = 3 };
@@ -191,8 +192,8 @@ bool build_mesh_topology(const double *nodes, int ntri_in, double curvature, dou
 // split-precision pair step (gb2_split.cu)
 void launch_pair_split(const Dev &D, cudaStream_t st, int shearupdate, int integrate, int fuse_next, int store_f,
                        size_t smem);
-void launch_tail_split(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                       int store_f);
+void launch_tail_split(const Dev &D, bool long_lists, int nblocks, cudaStream_t st, int shearupdate, int integrate,
+                       int fuse_next, int store_f);
 bool tri_neighbuild_host(const TriGeom &T, double rSphere, const double *c, double treshold);
 // Small page-locked host words (flags and counts read back from the device)
 // in 256-byte slots of a process-wide arena: locking host pages costs

@@ -1001,7 +1001,9 @@ __global__ void k_tail_list(Dev D)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= D.nlocal) return;
-    const bool tail = tail_atom(D, k, D.rnum[k], D.nnum[k]);
+    const int nr = D.rnum[k], nn = D.nnum[k];
+    const bool tail = tail_atom(D, k, nr, nn);
+    if (nr > 64 || nn > 64) atomicOr(D.status, ST_LONG_LISTS);
     D.tflag[k] = tail ? 1 : 0;
     if (tail) D.tail[atomicAdd(D.tailcnt, 1)] = k;
 }

@@ -17,11 +17,10 @@ void launch_pair_split(const Dev &D, cudaStream_t st, int shearupdate, int integ
     launch_pair_step<true>(D, 1, st, shearupdate, integrate, fuse_next, store_f, smem);
 }
 
-void launch_tail_split(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                       int store_f)
+void launch_tail_split(const Dev &D, bool long_lists, int nblocks, cudaStream_t st, int shearupdate, int integrate,
+                       int fuse_next, int store_f)
 {
-    if (D.rolling) launch_pair_tail<true, true>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f);
-    else launch_pair_tail<false, true>(D, nblocks, st, shearupdate, integrate, fuse_next, store_f);
+    launch_pair_tail<true>(D, long_lists, nblocks, st, shearupdate, integrate, fuse_next, store_f);
 }
 
 }  // namespace gb2

@@ -113,11 +113,8 @@ __device__ __forceinline__ void eval_item(const Dev &D, int kk, int other, int s
 // entries of four chunks are in flight together; one lane taking the entries
 // one by one (a 3 mm sphere in a bed of 0.3 mm spheres has hundreds) set the
 // whole step's time.  Out of line, as inlined it would take part in the tail
-// kernel's register allocation; the call has its price too (the tail kernel
-// keeps more of its state in local memory around it than it does without, and
-// took 41.6 us a launch instead of 39.7 on the packed 1M hopper, which has no
-// such atom).  FP64 in both precisions, records from L2 (called before the
-// wait).
+// kernel's register allocation (the call costs spills as well, see k_pair_tail).
+// FP64 in both precisions, records from L2 (called before the wait).
 constexpr int kLongList = kTailAtoms * 64;
 
 template <bool ROLLING>
@@ -573,7 +570,12 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
 // fix, walls not yet done evaluated now, then final_integrate and the
 // fused next initial_integrate.  Every atom's end of step touches only that
 // atom's records, so the result is bit for bit that of one kernel.
-template <bool ROLLING, bool SPLIT>
+// LONG: some atom of the context has more than 64 entries on a side.  The call
+// of long_atom costs the kernel 1,600 bytes of spills, taken or not (a step of the
+// 6,000-sphere hopper 19.6 us against 18.5 without it, of the 40,000-sphere drum
+// 24.6 against 23.8), so contexts without such an atom, as most are, run the
+// kernel that does not hold it.
+template <bool ROLLING, bool SPLIT, bool LONG>
 __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ Dev D, int shearupdate, int integrate, int fuse_next,
                                                       int store_f)
 {
@@ -612,20 +614,21 @@ __global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ De
                 }
             }
         }
-        const bool serial = nr > 64 || nn > 64;
+        const bool serial = LONG && (nr > 64 || nn > 64);
         // long lists, also before the wait: their sums need nothing of the pair step
         ContactOut lacc;
         for (int c = 0; c < 3; c++) lacc.F[c] = lacc.T[c] = 0.0;
-        for (unsigned m = __ballot_sync(0xffffffffu, own && serial); m; m &= m - 1u) {
-            const int src = __ffs(m) - 1;
-            ContactOut a;
-            long_atom<ROLLING>(D, __shfl_sync(0xffffffffu, i, src), __shfl_sync(0xffffffffu, nr, src),
-                               __shfl_sync(0xffffffffu, nn, src), upd, s_sp[wid], a);
-            if (lane == src) {
-                lacc = a;
-                if (upd) D.prevmask[i] = ~0ull;   // every own slot written this step
+        if constexpr (LONG)
+            for (unsigned m = __ballot_sync(0xffffffffu, own && serial); m; m &= m - 1u) {
+                const int src = __ffs(m) - 1;
+                ContactOut a;
+                long_atom<ROLLING>(D, __shfl_sync(0xffffffffu, i, src), __shfl_sync(0xffffffffu, nr, src),
+                                   __shfl_sync(0xffffffffu, nn, src), upd, s_sp[wid], a);
+                if (lane == src) {
+                    lacc = a;
+                    if (upd) D.prevmask[i] = ~0ull;   // every own slot written this step
+                }
             }
-        }
         const double vi[3] = {vi4.x, vi4.y, vi4.z}, wi[3] = {wi4.x, wi4.y, wi4.z};
         // walls before the wait: atoms with one wall fix at work
         bool early = own && !serial && nwork == 1;
@@ -743,11 +746,15 @@ inline cudaError_t launch_pair_step(const Dev &D, int lanes, cudaStream_t st, in
 }
 
 // Host side: the tail kernel of the pair step launched just before it.
-template <bool ROLLING, bool SPLIT>
-inline cudaError_t launch_pair_tail(const Dev &D, int nblocks, cudaStream_t st, int shearupdate, int integrate,
-                                    int fuse_next, int store_f)
+template <bool SPLIT>
+inline cudaError_t launch_pair_tail(const Dev &D, bool long_lists, int nblocks, cudaStream_t st, int shearupdate,
+                                    int integrate, int fuse_next, int store_f)
 {
-    return launch_dependent(k_pair_tail<ROLLING, SPLIT>, nblocks, 0, st, D, shearupdate, integrate, fuse_next, store_f);
+    auto kernel = k_pair_tail<false, SPLIT, false>;
+    if (D.rolling && long_lists) kernel = k_pair_tail<true, SPLIT, true>;
+    else if (D.rolling) kernel = k_pair_tail<true, SPLIT, false>;
+    else if (long_lists) kernel = k_pair_tail<false, SPLIT, true>;
+    return launch_dependent(kernel, nblocks, 0, st, D, shearupdate, integrate, fuse_next, store_f);
 }
 
 }  // namespace gb2
