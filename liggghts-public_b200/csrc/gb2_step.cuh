@@ -543,6 +543,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     ContactOut acc;
     pair_total<SPLIT>(as, kc, acc);
     if (!owns) return;
+    pk = ldrec(&D.pos[k]);   // again: the rounds need its registers (packed 1M hopper 260 -> 240 us/step)
     cp_async_wait();
     if (!serial) atom_hist_tail(D, k, prevm, mown, upd);
     if (tail) {   // finished by k_pair_tail from these pair sums
