@@ -22,12 +22,12 @@ from parity_util import assert_atoms_equal, assert_mesh_equal, assert_pairs_equa
 R, SKIN = 1e-3, 0.5e-3
 
 
-def _strip(xs, ys, upright=False):
+def _strip(xs, ys, focus, upright=False):
     """Two triangles per cell of the grid xs x ys: on z = 0 facing up, or, upright, on y = 0 facing +y with
-    ys along z.  The middle row of cells comes last, in each row the cells at small x."""
+    ys along z.  The middle row of cells comes last, in each row the cells next to x = focus."""
     tris, rows = [], len(ys) - 1
     for b in sorted(range(rows), key=lambda b: -abs(2 * b - (rows - 1))):
-        for a in reversed(range(len(xs) - 1)):
+        for a in sorted(range(len(xs) - 1), key=lambda a: -abs(0.5 * (xs[a] + xs[a + 1]) - focus)):
             p = [(xs[a], ys[b]), (xs[a + 1], ys[b]), (xs[a + 1], ys[b + 1]), (xs[a], ys[b + 1])]
             q = [(x, 0.0, y) if upright else (x, y, 0.0) for x, y in p]
             for t in ((0, 1, 2), (0, 2, 3)):
@@ -46,8 +46,9 @@ def _scene(n=12, walls="floor"):
     vel = np.zeros((n, 3))
     vel[:, 0] = 1.0 + rng.uniform(-0.01, 0.01, n)
     vel[:, 1] = -1e-3
-    floor = {"kind": "wall_mesh", "nodes": _strip(xs, ys), "wall_type": 1, "curvature": 0.0}
-    upright = {"kind": "wall_mesh", "nodes": _strip(np.arange(-0.04, 0.02, 0.9e-3), np.arange(-2e-3, 4.1e-3, 2e-3), True),
+    focus = coarse[-1] - R   # where the first sphere is when its list first outgrows 32
+    floor = {"kind": "wall_mesh", "nodes": _strip(xs, ys, focus), "wall_type": 1, "curvature": 0.0}
+    upright = {"kind": "wall_mesh", "nodes": _strip(np.arange(-0.04, 0.02, 0.9e-3), np.arange(-2e-3, 4.1e-3, 2e-3), focus, True),
                "wall_type": 1, "curvature": 0.0}
     meshes = {"floor": [floor], "floor_first": [floor, upright], "floor_last": [upright, floor]}[walls]
     sc = S.hopper(n=8, n_theta=12, n_z=4, seed=1)
@@ -88,19 +89,22 @@ def _check(e, o, sc):
 
 
 def test_scene_reaches_the_growth():
-    """What the GPU tests rest on, by the oracle and geometry alone: at the start no sphere is near more than
-    32 triangles of any mesh; later one is near 33 to 64 of the floor's and touches one of the last."""
+    """What the GPU tests rest on, by the oracle and geometry alone: at the start no sphere lists more than 32
+    triangles of any mesh; the first that does touches one beyond the 32nd, and so does some sphere at the end."""
     sc = _scene(walls="floor_last")
     o = oracle.Oracle(sc)
     o.setup()
     up, fl = (sc["fixes"][k]["nodes"] for k in _meshes(sc))
-    before = [_close(fl, x)[0] for x in o.atoms()["x"]]
-    assert max(before) <= 32 and max(_close(up, x)[0] for x in o.atoms()["x"]) <= 32
+    assert max(_close(n, x)[0] for n in (up, fl) for x in o.atoms()["x"]) <= 32
     assert len(o.mesh_contacts(2)["tag"]) > 0
-    o.run(3000)
-    x = o.atoms()["x"]
-    cnt, rank = np.array([_close(fl, p) for p in x]).T
-    assert 32 < cnt.max() <= 64 and (rank[cnt > 32] >= 32).any()
+    first = None
+    for _ in range(60):
+        o.run(50)
+        cnt, rank = np.array([_close(fl, p) for p in o.atoms()["x"]]).T
+        if first is None and cnt.max() > 32:
+            first = rank[cnt.argmax()]
+        assert cnt.max() <= 64
+    assert first >= 32 and (rank >= 32).any()
     assert len(o.mesh_contacts(2)["tag"]) > 0 and len(o.mesh_contacts(1)["tag"]) > 0
 
 
