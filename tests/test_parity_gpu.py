@@ -134,7 +134,8 @@ def test_silo_cylinder_wall_and_linear_piston():
 def test_bidisperse_long_lists_serial_path():
     """Two 3 mm spheres buried in a bed of 0.3 mm ones: each has ~177
     neighbour-list pairs, more than 64 on a side, so its pairs are evaluated
-    serially in the reference order by the tail kernel; bit for bit."""
+    by a warp of the tail kernel and added in the reference order; bit for
+    bit."""
     import granb200
     sc = S.bidisperse_bed()
     e, o = _pair(sc)
