@@ -293,60 +293,12 @@ struct WarpItems {
     int cnt, excl, total;
 };
 
-__device__ __forceinline__ WarpItems warp_items(unsigned long long mask)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    WarpItems it;
-    it.cnt = __popcll(mask);
-    int x = it.cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(FULL, x, o);
-        if (lane >= o) x += y;
-    }
-    it.excl = x - it.cnt;
-    it.total = __shfl_sync(FULL, x, 31);
-    return it;
-}
-
 // Index stream loads: read once per step, evict-first so they do not push
 // the neighbour records out of L2
 __device__ __forceinline__ int ld_stream(const int *p) { return __ldcs(p); }
 
-// Screening of the j-side (rev) and own (nbr) entries of one atom in one
-// loop: per round two indices of each list, then four independent record
-// gathers, then the distance tests.  Both lists are <= 64 entries here.
-__device__ __forceinline__ void screen_both(const Dev &D, int k, int nr, int nn, const dbl4 &pk,
-                                            unsigned long long &mrev, unsigned long long &mown)
-{
-    const int cap = D.cap;
-    const int n = max(nr, nn);
-    // the indices of the next pair of entries are requested while this
-    // pair's records are in flight (one dependent round trip per pair)
-    int a0 = (0 < nr) ? ld_stream(&D.rev[k]) : k;
-    int a1 = (1 < nr) ? ld_stream(&D.rev[cap + k]) : k;
-    int b0 = (0 < nn) ? ld_stream(&D.nbr[k]) : k;
-    int b1 = (1 < nn) ? ld_stream(&D.nbr[cap + k]) : k;
-    for (int t = 0; t < n; t += 2) {
-        const dbl4 qa0 = ldrec(&D.pos[a0]);
-        const dbl4 qa1 = ldrec(&D.pos[a1]);
-        const dbl4 qb0 = ldrec(&D.pos[b0]);
-        const dbl4 qb1 = ldrec(&D.pos[b1]);
-        const int u = t + 2;
-        a0 = (u < nr) ? ld_stream(&D.rev[u * cap + k]) : k;
-        a1 = (u + 1 < nr) ? ld_stream(&D.rev[(u + 1) * cap + k]) : k;
-        b0 = (u < nn) ? ld_stream(&D.nbr[u * cap + k]) : k;
-        b1 = (u + 1 < nn) ? ld_stream(&D.nbr[(u + 1) * cap + k]) : k;
-        if (t < nr && touching(pk, qa0)) mrev |= 1ull << t;
-        if (t + 1 < nr && touching(pk, qa1)) mrev |= 1ull << (t + 1);
-        if (t < nn && touching(pk, qb0)) mown |= 1ull << t;
-        if (t + 1 < nn && touching(pk, qb1)) mown |= 1ull << (t + 1);
-    }
-}
-
-// Screening that also lists the warp's touching entries in shared memory,
-// so the contact rounds read each item's partner and slot there instead of
+// Screening of the j-side (rev) and own (nbr) entries of a warp's atoms in one
+// loop, listing the touching entries in shared memory, so the contact rounds read each item's partner and slot there instead of
 // gathering the list index again: lrev holds the j-side entries, lown the
 // own entries, each as {other atom, owner lane | slot << 8} in the order the
 // owner's sum takes them (every atom's rev entries by r, then its own entries
@@ -368,10 +320,9 @@ __device__ __forceinline__ void list_append(int2 *list, int cap, int &n, bool ta
     n += __popc(m);
 }
 
-//
 // U entries of each list are in flight together (their records are requested,
 // then the next U indices, then the tests): four in FP64 (against two: hopper
-// of 1M 255 -> 253 us/step, bed of 2M 818 -> 808), two in split precision,
+// of 1M 255 -> 250 us/step, bed of 2M 814 -> 804), two in split precision,
 // whose 80 registers do not hold eight records (205 -> 274), in the loop its
 // contact arithmetic was always compiled beside (contraction, and with it the
 // last bits, depend on the code around).

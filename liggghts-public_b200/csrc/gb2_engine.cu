@@ -1080,7 +1080,8 @@ int do_build(gb2_ctx *c)
         if (clear_status(c)) return GB2_ERR_CUDA;
         CK(cudaMemsetAsync(c->rnum.p, 0, sizeof(int) * c->cap, c->st));
         D = make_dev(c);
-        // eight lanes per atom where the bins hold more than ~4 atoms on average
+        // eight lanes per atom where the bins hold more than ~4 atoms on average,
+        // empty bins counted: a crowded region in a mostly empty box keeps one lane
         if ((long)nall >= 4l * c->mbins)
             k_build_list<8><<<nblk(8l * c->nlocal), kBlock, 0, c->st>>>(D);
         else

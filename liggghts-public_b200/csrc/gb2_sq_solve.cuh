@@ -23,7 +23,7 @@
 // particle packing (20 steps, ~22,000 solves each) went from 2.27 ms to
 // 0.52 ms, one of 2,000 particles (60 steps) from 0.67 ms to 0.17 ms, with the
 // same iteration and solve counts.  168 registers (3 blocks per SM) keep the
-// state of a solve out of local memory but for ~20 doubles; a group of 16
+// state of a solve out of local memory but for some 25 doubles; a group of 16
 // lanes would only shorten the golden-section pairs.
 #pragma once
 

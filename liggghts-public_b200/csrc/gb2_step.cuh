@@ -445,8 +445,8 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
     // entries (all lanes take part in the list ballots)
     int nlrev = 0, nlown = 0;
     int2 *lrev = reinterpret_cast<int2 *>(pair_dyn) + (size_t)wid * 2 * D.item_cap, *lown = lrev + D.item_cap;
-    const bool listed = screen_list<G, SPLIT ? 2 : 4>(D, k, (valid && !serial) ? nr : 0, (valid && !serial) ? nn : 0, pk, mrev, mown,
-                                       lrev, lown, nlrev, nlown);
+    const bool listed = screen_list<G, SPLIT ? 2 : 4>(D, k, (valid && !serial) ? nr : 0, (valid && !serial) ? nn : 0,
+                                                      pk, mrev, mown, lrev, lown, nlrev, nlown);
     if (!listed && lane == 0 && D.item_cap > 0) atomicAdd(&D.need[4], 1);   // lists too short: counted for the host
     // FP64 path: plain in-order sums (bit-exact).  Split path: FP32 sums of
     // the FP32 pair contributions with Kahan compensation kc.
@@ -572,13 +572,13 @@ __global__ void __launch_bounds__(128, MINB) k_pair_step(Dev D, int shearupdate,
 // fused next initial_integrate.  Every atom's end of step touches only that
 // atom's records, so the result is bit for bit that of one kernel.
 // LONG: some atom of the context has more than 64 entries on a side.  The call
-// of long_atom costs the kernel 1,600 bytes of spills, taken or not (a step of the
-// 6,000-sphere hopper 19.6 us against 18.5 without it, of the 40,000-sphere drum
-// 24.6 against 23.8), so contexts without such an atom, as most are, run the
-// kernel that does not hold it.
+// of long_atom costs the kernel 1,600 bytes of spills, taken or not (a launch on
+// the timed 1M hopper 30.4 us against 27.6 without it, a step of the 6,000-sphere
+// hopper 20.0 against 18.9, of the 40,000-sphere drum 24.6 against 24.3), so
+// contexts without such an atom, as most are, run the kernel that does not hold it.
 template <bool ROLLING, bool SPLIT, bool LONG>
-__global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ Dev D, int shearupdate, int integrate, int fuse_next,
-                                                      int store_f)
+__global__ void __launch_bounds__(128, 4) k_pair_tail(const __grid_constant__ Dev D, int shearupdate, int integrate,
+                                                      int fuse_next, int store_f)
 {
     __shared__ int s_sp[4][kTailAtoms * 64];            // slot partners of the warp's atoms (mesh walls)
     __shared__ WallRec s_rec[4][kTailAtoms][kWallRec];  // wall-contact records of the warp's atoms
@@ -717,13 +717,14 @@ inline cudaError_t launch_dependent(Kernel kernel, int nblocks, size_t smem, cud
 }
 
 // The pair step with one or (FP64) two lanes per atom.  Registers: FP64 takes 4 blocks
-// per SM (128 registers, no spill): 5 blocks (96) spill 20 doubles through the
-// L1 that the gathers need, 3 leave too few warps (hopper of 1M 253, 267 and
-// 307 us/step, bed of 2M 847, 907 and 847).  Split precision fits 6 blocks (80):
-// 206 us/step against 209 with 5 and 240 with 4.
+// per SM (128 registers, at most 4 bytes of spills): 5 blocks (96) spill 20
+// doubles through the L1 that the gathers need, 3 leave too few warps (hopper of
+// 1M 253, 267 and 307 us/step, bed of 2M 847, 907 and 847).  Split precision takes
+// 6 blocks (80, with 40 to 68 bytes spilled): 206 us/step against 209 with 5 and
+// 240 with 4.
 template <bool ROLLING, bool SPLIT, bool ONE>
-inline cudaError_t launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                            int store_f, size_t smem)
+inline cudaError_t launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate,
+                                   int fuse_next, int store_f, size_t smem)
 {
     auto kernel = k_pair_step<ROLLING, SPLIT ? 6 : 4, SPLIT, ONE, 1>;
     if constexpr (!SPLIT) {
@@ -734,8 +735,8 @@ inline cudaError_t launch_pair_one(const Dev &D, int lanes, cudaStream_t st, int
 }
 
 template <bool SPLIT>
-inline cudaError_t launch_pair_step(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate, int fuse_next,
-                             int store_f, size_t smem)
+inline cudaError_t launch_pair_step(const Dev &D, int lanes, cudaStream_t st, int shearupdate, int integrate,
+                                    int fuse_next, int store_f, size_t smem)
 {
     if (D.rolling && D.ntypes == 1)
         return launch_pair_one<true, SPLIT, true>(D, lanes, st, shearupdate, integrate, fuse_next, store_f, smem);
